@@ -124,13 +124,13 @@ typedef struct rm_config {
 typedef struct rm_stats {
   uint64_t path_samples;    /* (pixel, sample) radiance estimates taken */
   uint64_t rays;            /* traversal queries (closest + any-hit) */
-  uint64_t nodes_visited;   /* BVH child-pair records fetched (64 B each) */
+  uint64_t nodes_visited;   /* BVH records fetched, in units of bvh_node_bytes (a 4-wide node of 128 B counts two) */
   uint64_t tris_tested;     /* Moller-Trumbore tests (48 B records) */
   uint64_t frames;
   uint64_t kernel_launches; /* this library's kernels launched by frame calls */
   uint32_t device_error;    /* last nonzero device error word, 0 if none */
   uint32_t kernel_chain;    /* 1 = render_paths, 8/32 = lane kernels, 2 = ReSTIR chain */
-  uint32_t bvh_node_bytes;  /* bytes of one node visit: 80 (8-wide compressed BVH) or 64 (binary) */
+  uint32_t bvh_node_bytes;  /* bytes of one counted node: 80 (8-wide compressed BVH) or 64 (binary and 4-wide) */
   uint32_t bvh_builds;      /* device BVH builds of the resident scene since the context was created */
   uint32_t bvh_refits;      /* device BVH refits of the resident scene since the context was created */
   uint32_t bvh_kept;        /* uploads of the resident scene with unchanged triangles: BVH kept, not rebuilt */

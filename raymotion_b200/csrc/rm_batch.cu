@@ -217,14 +217,15 @@ __device__ __forceinline__ TraceResult bt_traverse(const Scene& s, float ox, flo
                                                    float dz, float tmax, uint32_t* err, uint32_t& nodes,
                                                    uint32_t& tests) {
   if (kWide) return traverse_any<kAnyHit>(s, ox, oy, oz, dx, dy, dz, tmax, err, nodes, tests);
-  return traverse<kAnyHit>(s, ox, oy, oz, dx, dy, dz, tmax, err, nodes, tests);
+  return traverse_quad<kAnyHit>(s, ox, oy, oz, dx, dy, dz, tmax, err, nodes, tests);
 }
 
-// Ten 128-thread blocks per SM (48 registers, ~100 bytes of spills; nine at
-// 55), and three 256-thread k_bt_shade blocks (80 registers, against two at
-// 113): batched config-3 rendering 914 against 866 M path samples/s.
+// Seven 128-thread blocks per SM (72 registers, no spills) for the 4-wide
+// traversal: a batch of eight uneven images 24.5 ms against 24.9 at six, 25.2
+// at eight and 25.7 at ten (48 registers); the binary records took 25.2 at
+// eight.  Three 256-thread k_bt_shade blocks (80 registers, against two at 113).
 template <bool kShadowRays, bool kWide>
-__global__ void __launch_bounds__(128, 10) k_bt_trace(BtBatch b, BtState w, BtQueues q, unsigned long long* ctr,
+__global__ void __launch_bounds__(128, 7) k_bt_trace(BtBatch b, BtState w, BtQueues q, unsigned long long* ctr,
                                                   uint32_t* err) {
   const int n = q.counts[kShadowRays ? kBtShd : kBtExt];
   const int* queue = kShadowRays ? q.shd : q.ext;

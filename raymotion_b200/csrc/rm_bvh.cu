@@ -394,6 +394,7 @@ cudaError_t refit_bvh(const rm_triangle* d_tris, DevBvh& bvh, cudaStream_t st) {
                                                        bvh.parents.as<int32_t>(), bvh.counters.as<int>(),
                                                        bvh.n_records);
   e = cudaGetLastError();
+  if (e == cudaSuccess) e = refit_quads(bvh, st);
   if (e != cudaSuccess) return e;
   return pack_tgeo(d_tris, bvh, st);
 }
@@ -436,6 +437,7 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
     k_single_leaf<<<1, 1, 0, st>>>(d_tris, n, b.records.as<float4>(), b.parents.as<int>(), b.order.as<int>());
     RM_TRY(cudaGetLastError());
     b.max_depth = 1;
+    RM_TRY(build_quads(b, st));
     return pack_tgeo(d_tris, b, st);
   }
   const int ni = n - 1;
@@ -487,6 +489,7 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(cudaMemcpyAsync(&b.max_depth, b.depth.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
   RM_TRY(cudaStreamSynchronize(st));
   if (b.max_depth > kStack) { err = "device BVH deeper than the traversal stack"; return cudaErrorInvalidValue; }
+  RM_TRY(build_quads(b, st));
   return pack_tgeo(d_tris, b, st);
 }
 
@@ -817,6 +820,7 @@ cudaError_t build_ploc(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(cudaStreamSynchronize(st));
   if (b.max_depth > kStack) { err = "device BVH deeper than the traversal stack"; return cudaErrorInvalidValue; }
   b.n_records = n - 1;
+  RM_TRY(build_quads(b, st));
   return pack_tgeo(d_tris, b, st);
 }
 
@@ -911,6 +915,10 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
           cudaSuccess ||
       (e = cudaStreamSynchronize(st)) != cudaSuccess) {
     err = std::string("BVH upload failed: ") + cudaGetErrorString(e);
+    return false;
+  }
+  if ((e = build_quads(out, st)) != cudaSuccess) {
+    err = std::string("BVH collapse failed: ") + cudaGetErrorString(e);
     return false;
   }
   return true;

@@ -82,7 +82,7 @@ struct DevScene {
   void release() {
     for (DevBuf* b : {&tri_mat, &mats, &tris, &tris_in, &lights, &cdf, &texels, &lrec, &guide, &bvh.records, &bvh.parents, &bvh.counters,
                       &bvh.order, &bvh.tgeo, &bvh.keys, &bvh.keys_alt, &bvh.vals_alt, &bvh.knodes, &bvh.kbox,
-                      &bvh.kcount, &bvh.ranges, &bvh.temp, &bvh.bounds, &bvh.depth, &bvh.wnodes, &bvh.wtgeo,
+                      &bvh.kcount, &bvh.ranges, &bvh.temp, &bvh.bounds, &bvh.depth, &bvh.quads, &bvh.qroots, &bvh.wnodes, &bvh.wtgeo,
                       &bvh.wq})
       b->release();
     if (bvh.h_wcnt) cudaFreeHost(bvh.h_wcnt);

@@ -13,7 +13,10 @@
 //    the Efficiency of Ray Traversal on GPUs", HPG 2009): each internal node
 //    holds both children's boxes, 64 bytes = four 128-bit loads; a ray tests
 //    both children at once and descends into the nearer one first with a
-//    per-thread stack.
+//    per-thread stack (Trav: the wavefront traversal, ReSTIR generate and
+//    spatial reuse, the no-allocation query).
+//  * quads: the 4-wide BVH collapsed from them, 128 bytes per node (QTrav: the
+//    one-thread-per-path kernels, the batch traversal and the ray queries).
 //  * tris: the caller's packed 176-byte triangles, read only for the surface
 //    attributes of a confirmed hit and for light sampling.
 #pragma once
@@ -71,6 +74,9 @@ struct Scene {
   const float4* __restrict__ tgeo;
   const float4* __restrict__ nodes;
   int n_nodes;  // internal child-pair records; 0 = empty scene
+  // 4-wide BVH collapsed from `nodes` (rm_quad.cu), 8 x float4 per node: what
+  // QTrav reads (null: only the binary records, read by Trav)
+  const float4* __restrict__ quads;
   const int32_t* __restrict__ lights;
   const float* __restrict__ cdf;
   int n_lights;
@@ -363,6 +369,137 @@ struct Trav {
   }
 };
 
+// Traversal of the 4-wide BVH (rm_quad.cu).  A node is one 128-byte line:
+// the four children's bounds (lo.x, hi.x, lo.y, hi.y, lo.z, hi.z, a float4
+// each) and their words (8-bit triangle count / 24-bit link, the stack entry;
+// 0: no child).  A step visits nodes until a leaf is pending, going on into the
+// nearest hit child and pushing the others, tests that leaf, and pops the next
+// subtree.
+//
+// A ray fetches half as many dependent records as in the binary BVH (12.3
+// against 25.2 on the 720p frame's extension rays) for about the same
+// instructions, which pays where registers are no limit: the plain frame
+// (150 k triangles, 1280x720, 16 spp) 18.9 against 20.7 ms through the binary
+// records, the plain adjoint step (512x512, 32 spp) 46.9 against 50.8, the
+// tail of the 720p ReSTIR frame 69 against 76 ms (three parts summed), a million
+// closest-hit queries 461 against 511 us (leaves of two triangles on both
+// sides).  The seven 128-bit loads in flight spill at the 48 registers of
+// k_wf_trace2 and k_restir_generate (frame 119 against 115 ms, generate 14.4
+// against 12.6), which keep the binary records.
+//
+// Pushes store all four words and advance the stack only for the hit ones: as
+// branches they split the warp (94 M against 52 M warp instructions for one
+// wave).  Entry distances on the stack, to cull at the pop, saved 2 % of the
+// visits and doubled the stack's lines (138 against 119 ms).
+//
+// Box test: Trav's, with the near and far bounds picked by the sign of i when
+// the node is read (near is lo for i >= 0) instead of by min / max; an axis
+// whose o i overflows culls nothing, as there.
+constexpr int kQuadStack = 3 * kStack / 2 + 4;  // at most three pushed per two binary levels
+
+struct QTrav {
+  float ox, oy, oz, dx, dy, dz, ix, iy, iz;
+  float cxn, cxf, cyn, cyf, czn, czf;  // slab addends of the near / far bound per axis
+  TraceResult r;
+  int sx, sy, sz;  // 0: near is lo, 1: near is hi
+  int sp;
+  uint32_t cur;  // the pending subtree's word
+
+  static __device__ __forceinline__ void addends(float o, float i, float& near_, float& far_) {
+    const float oi = o * i;
+    const float m = fabsf(oi) * 0x1p-21f;
+    const bool finite = fabsf(oi) <= 3.4028234663852886e38f;
+    const float inf = __int_as_float(0x7f800000);
+    near_ = finite ? -oi - m : -inf;
+    far_ = finite ? -oi + m : inf;
+  }
+
+  __device__ __forceinline__ void init(float ox_, float oy_, float oz_, float dx_, float dy_, float dz_, float tmax) {
+    ox = ox_; oy = oy_; oz = oz_; dx = dx_; dy = dy_; dz = dz_;
+    ix = 1.0f / (dx == 0.0f ? 1e-30f : dx);
+    iy = 1.0f / (dy == 0.0f ? 1e-30f : dy);
+    iz = 1.0f / (dz == 0.0f ? 1e-30f : dz);
+    addends(ox, ix, cxn, cxf);
+    addends(oy, iy, cyn, cyf);
+    addends(oz, iz, czn, czf);
+    sx = ix >= 0.0f ? 0 : 1; sy = iy >= 0.0f ? 0 : 1; sz = iz >= 0.0f ? 0 : 1;
+    r = TraceResult{tmax, -1, 0.f, 0.f};
+    sp = 0;
+    cur = 0u;  // the root
+  }
+
+  // Pop the next pending subtree; true when none is left.
+  __device__ __forceinline__ bool pop(const uint32_t* stack) {
+    if (sp == 0) return true;
+    cur = stack[--sp];
+    return false;
+  }
+
+  // Box-test the four children of node `cur` and move on.  True when nothing
+  // is left (or the stack overflowed, flagged in err).
+  __device__ __forceinline__ bool visit(const Scene& s, uint32_t* stack, uint32_t* err, uint32_t& n_nodes) {
+    if (bad_index(cur, s.n_nodes, err, kSiteNode)) return pop(stack);
+    n_nodes += 2;  // one node is two 64-byte records
+    const float4* n = s.quads + size_t(cur) * 8;
+    const float4 nx = __ldg(n + sx), fx = __ldg(n + (sx ^ 1));
+    const float4 ny = __ldg(n + 2 + sy), fy = __ldg(n + 2 + (sy ^ 1));
+    const float4 nz = __ldg(n + 4 + sz), fz = __ldg(n + 4 + (sz ^ 1));
+    const uint4 w = __ldg(reinterpret_cast<const uint4*>(n + 6));
+    const float t0 = fmax3(__fmaf_rn(nx.x, ix, cxn), __fmaf_rn(ny.x, iy, cyn), fmaxf(__fmaf_rn(nz.x, iz, czn), 0.0f));
+    const float t1 = fmax3(__fmaf_rn(nx.y, ix, cxn), __fmaf_rn(ny.y, iy, cyn), fmaxf(__fmaf_rn(nz.y, iz, czn), 0.0f));
+    const float t2 = fmax3(__fmaf_rn(nx.z, ix, cxn), __fmaf_rn(ny.z, iy, cyn), fmaxf(__fmaf_rn(nz.z, iz, czn), 0.0f));
+    const float t3 = fmax3(__fmaf_rn(nx.w, ix, cxn), __fmaf_rn(ny.w, iy, cyn), fmaxf(__fmaf_rn(nz.w, iz, czn), 0.0f));
+    const float f0 = fmin3(__fmaf_rn(fx.x, ix, cxf), __fmaf_rn(fy.x, iy, cyf), fminf(__fmaf_rn(fz.x, iz, czf), r.t));
+    const float f1 = fmin3(__fmaf_rn(fx.y, ix, cxf), __fmaf_rn(fy.y, iy, cyf), fminf(__fmaf_rn(fz.y, iz, czf), r.t));
+    const float f2 = fmin3(__fmaf_rn(fx.z, ix, cxf), __fmaf_rn(fy.z, iy, cyf), fminf(__fmaf_rn(fz.z, iz, czf), r.t));
+    const float f3 = fmin3(__fmaf_rn(fx.w, ix, cxf), __fmaf_rn(fy.w, iy, cyf), fminf(__fmaf_rn(fz.w, iz, czf), r.t));
+    const bool h0 = w.x != 0u && !(t0 > f0 * kFmaBoxSlack);
+    const bool h1 = w.y != 0u && !(t1 > f1 * kFmaBoxSlack);
+    const bool h2 = w.z != 0u && !(t2 > f2 * kFmaBoxSlack);
+    const bool h3 = w.w != 0u && !(t3 > f3 * kFmaBoxSlack);
+    // nearest hit child: the entry distances are >= 0, so their bits order as
+    // integers; the low two bits carry the slot
+    const uint32_t none = 0xFFFFFFFFu;
+    const uint32_t k0 = h0 ? (__float_as_uint(t0) & ~3u) : none;
+    const uint32_t k1 = h1 ? ((__float_as_uint(t1) & ~3u) | 1u) : none;
+    const uint32_t k2 = h2 ? ((__float_as_uint(t2) & ~3u) | 2u) : none;
+    const uint32_t k3 = h3 ? ((__float_as_uint(t3) & ~3u) | 3u) : none;
+    const uint32_t m = min(min(k0, k1), min(k2, k3));
+    if (m == none) return pop(stack);
+    if (sp > kQuadStack - 4) { atomicOr(err, kErrStack); return true; }
+    stack[sp] = w.x; sp += int(h0 && k0 != m);
+    stack[sp] = w.y; sp += int(h1 && k1 != m);
+    stack[sp] = w.z; sp += int(h2 && k2 != m);
+    stack[sp] = w.w; sp += int(h3 && k3 != m);
+    cur = (m & 2u) ? ((m & 1u) ? w.w : w.z) : ((m & 1u) ? w.y : w.x);
+    return false;
+  }
+
+  template <bool kAnyHit>
+  __device__ __forceinline__ bool step(const Scene& s, uint32_t* stack, uint32_t* err, uint32_t& n_nodes,
+                                       uint32_t& n_tests) {
+    return step_rt(s, stack, err, n_nodes, n_tests, kAnyHit);
+  }
+
+  // step() with the any-hit rule as a run-time flag: lanes of one warp that
+  // trace closest-hit and any-hit rays then run the same instructions.
+  __device__ __forceinline__ bool step_rt(const Scene& s, uint32_t* stack, uint32_t* err, uint32_t& n_nodes,
+                                          uint32_t& n_tests, bool any_hit) {
+    if (s.n_nodes == 0) return true;
+    while (cur < (1u << 24))
+      if (visit(s, stack, err, n_nodes)) return true;
+    // leaf: Moller-Trumbore, pathtrace.metal:150-158
+    int first = int(cur & 0xFFFFFFu), count = int(cur >> 24);
+    if (kChecked && (bad_index(first, s.n_tris, err, kSiteLeaf) ||
+                     bad_index(first + count - 1, s.n_tris, err, kSiteLeaf)))
+      count = 0;
+    n_tests += uint32_t(count);
+    for (int k = 0; k < count; ++k)
+      if (test_triangle(s.tgeo + size_t(first + k) * 3, ox, oy, oz, dx, dy, dz, r) && any_hit) return true;
+    return pop(stack);
+  }
+};
+
 // Traversal of the 8-wide compressed BVH built by rm_wide.cu.  A node is 5 x
 // float4: origin p (3 floats), the three scale exponents and the mask of
 // internal children (4 bytes), the index of its first internal child node and
@@ -443,7 +580,7 @@ struct WTrav {
     // A child's slab on axis a is t = q s_a i_a + (p_a - o_a) i_a, one fma per
     // bound from the per-node base (p_a - o_a) i_a and the exact product
     // s_a i_a (s_a is a power of two).  Its rounding differs from the base
-    // test's (L - o) i (Trav), so the near bound's base is lowered and the far
+    // test's (L - o) i (QTrav), so the near bound's base is lowered and the far
     // bound's raised by m_a = |i_a| 2^-20 (|p_a - o_a| + 256 s_a + |p_a|),
     // rounded outward: m_a exceeds the sum of both forms' rounding errors and
     // of the decoded bound's half ulp, so every box the base test accepts
@@ -506,14 +643,14 @@ struct WTrav {
   }
 };
 
-// One ray through the binary BVH (always built; the megakernels trace here,
-// so that the wide traversal's registers never count against them).
+// One ray through the 4-wide BVH (always built; the megakernels trace here, so
+// that the wide traversal's registers never count against them).
 template <bool kAnyHit>
-__device__ __forceinline__ TraceResult traverse(const Scene& s, float ox, float oy, float oz, float dx, float dy,
+__device__ __forceinline__ TraceResult traverse_quad(const Scene& s, float ox, float oy, float oz, float dx, float dy,
                                                 float dz, float tmax, uint32_t* err, uint32_t& n_nodes,
                                                 uint32_t& n_tests) {
-  Trav t;
-  int stack[kStack];
+  QTrav t;
+  uint32_t stack[kQuadStack];
   t.init(ox, oy, oz, dx, dy, dz, tmax);
   while (!t.step<kAnyHit>(s, stack, err, n_nodes, n_tests)) {
   }
@@ -533,13 +670,28 @@ __device__ __forceinline__ TraceResult traverse_rt(const Scene& s, float ox, flo
   return t.r;
 }
 
-// One ray through the 8-wide BVH when the scene has one, else the binary BVH
-// (the ray-query entry point; the wavefront trace kernels pick WTrav or Trav
+// One ray through the binary records (Trav).
+template <bool kAnyHit>
+__device__ __forceinline__ TraceResult traverse(const Scene& s, float ox, float oy, float oz, float dx, float dy,
+                                                 float dz, float tmax, uint32_t* err, uint32_t& n_nodes,
+                                                 uint32_t& n_tests) {
+  Trav t;
+  int stack[kStack];
+  t.init(ox, oy, oz, dx, dy, dz, tmax);
+  while (!t.step<kAnyHit>(s, stack, err, n_nodes, n_tests)) {
+  }
+  return t.r;
+}
+
+// One ray through the 8-wide BVH when the scene has one, else the 4-wide BVH
+// (the ray-query entry point; the wavefront trace kernels pick WTrav or QTrav
 // per launch instead).  Both give the same hits.
 template <bool kAnyHit>
 __device__ __forceinline__ TraceResult traverse_any(const Scene& s, float ox, float oy, float oz, float dx, float dy,
                                                     float dz, float tmax, uint32_t* err, uint32_t& n_nodes,
                                                     uint32_t& n_tests) {
+  // the no-allocation query builds only the binary records
+  if (!s.quads) return traverse<kAnyHit>(s, ox, oy, oz, dx, dy, dz, tmax, err, n_nodes, n_tests);
   if (s.wnodes) {
     WTrav t;
     uint2 stack[kWideStack];
@@ -548,7 +700,7 @@ __device__ __forceinline__ TraceResult traverse_any(const Scene& s, float ox, fl
     }
     return t.r;
   }
-  return traverse<kAnyHit>(s, ox, oy, oz, dx, dy, dz, tmax, err, n_nodes, n_tests);
+  return traverse_quad<kAnyHit>(s, ox, oy, oz, dx, dy, dz, tmax, err, n_nodes, n_tests);
 }
 
 // ---------------------------------------------------------------- tracer
@@ -565,6 +717,12 @@ struct Tracer {
   __device__ __forceinline__ float U() { return rng.uniform01(); }
 
   __device__ __forceinline__ bool shadow(float ox, float oy, float oz, float dx, float dy, float dz, float dist) {
+    ++rays;
+    return traverse_quad<true>(s, ox, oy, oz, dx, dy, dz, dist, err, nodes, tests).tri >= 0;
+  }
+  // shadow() through the binary records, for kernels short of registers
+  __device__ __forceinline__ bool shadow_binary(float ox, float oy, float oz, float dx, float dy, float dz,
+                                                float dist) {
     ++rays;
     return traverse<true>(s, ox, oy, oz, dx, dy, dz, dist, err, nodes, tests).tri >= 0;
   }
@@ -589,7 +747,7 @@ struct Tracer {
   // pathtrace.metal:165-204
   __device__ __noinline__ Hit cast_ray(float ox, float oy, float oz, float dx, float dy, float dz, float dist) {
     ++rays;
-    TraceResult tr = traverse<false>(s, ox, oy, oz, dx, dy, dz, dist, err, nodes, tests);
+    TraceResult tr = traverse_quad<false>(s, ox, oy, oz, dx, dy, dz, dist, err, nodes, tests);
     return attributes(tr, ox, oy, oz, dx, dy, dz);
   }
 

@@ -131,12 +131,14 @@ __global__ void __launch_bounds__(256) k_render_paths(Scene s, Params p, uint64_
 
 __device__ __forceinline__ int gkind(const GBufSoA& g, uint32_t i) { return __float_as_int(g.pos_kind[i].w); }
 
-// K3 restir_generate (pathtrace.metal:817-917).  Ten 128-thread blocks per SM
-// (48 registers, ~360 bytes of spills): the 32 candidates' shadow rays are
-// latency-bound, and the extra warps outweigh the spills (13.1 / 13.3 against
-// 13.4 / 13.6 ms at eight blocks and 64 registers on the 720p frame; six
-// blocks at 80 registers, 15.0 ms).
-__global__ void __launch_bounds__(128, 10) k_restir_generate(Scene s, Params p, uint64_t seed, GBufSoA gb, ResSoA ri,
+// K3 restir_generate (pathtrace.metal:817-917).  ReSTIR scenes are opaque
+// (metal.mm:237), so visibility is a plain any-hit ray.  Eight 128-thread
+// blocks per SM (64 registers): the 32 candidates' shadow rays are
+// latency-bound, and without the transparent crossings' code the kernel spills
+// little there (12.6 ms on the 720p frame against 13.4 at ten blocks and 48
+// registers; with that code 13.4 at eight, 13.1 at ten).  Shadow rays go
+// through the binary records: the 4-wide nodes took 14.4 ms.
+__global__ void __launch_bounds__(128, 8) k_restir_generate(Scene s, Params p, uint64_t seed, GBufSoA gb, ResSoA ri,
                                                          unsigned long long* ctr, uint32_t* err) {
   const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t npix = uint32_t(p.width) * uint32_t(p.height);
@@ -156,7 +158,7 @@ __global__ void __launch_bounds__(128, 10) k_restir_generate(Scene s, Params p, 
     float rdx = tx * c.m0 + (ty * c.m1 + tz * c.m2);
     float rdy = tx * c.m3 + (ty * c.m4 + tz * c.m5);
     float rdz = tx * c.m6 + (ty * c.m7 + tz * c.m8);
-    Hit hit = pt.cast_alpha_ray(c.x, c.y, c.z, rdx, rdy, rdz, kFar);
+    Hit hit = pt.cast_ray(c.x, c.y, c.z, rdx, rdy, rdz, kFar);
     if (hit.tri >= 0) {
       float pnx = hit.nix, pny = hit.niy, pnz = hit.niz;
       float geom = hit.ngx * pnx + (hit.ngy * pny + hit.ngz * pnz);
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(128, 10) k_restir_generate(Scene s, Params p, 
                 ph = lum3(Fr, Fg, Fb);
                 if (ph > 0.0f) {
                   wu = ph / q;
-                  bool occ = pt.occluded(sox, soy, soz, dxn, dyn, dzn, dist - 0.003f);
+                  bool occ = pt.shadow_binary(sox, soy, soz, dxn, dyn, dzn, dist - 0.003f);
                   if (!occ) ws = wu;
                 }
               }
@@ -331,7 +333,7 @@ __global__ void __launch_bounds__(256, 3) k_restir_spatial(Scene s, Params p, ui
             float ph, dist, dxn, dyn, dzn;
             if (eval_at(H0, H1, H2, ph, dist, dxn, dyn, dzn) && ph > 0.0f) {
               float wu = ph * hsumWu / hph;
-              bool occ = pt.occluded(sox, soy, soz, dxn, dyn, dzn, dist - 0.003f);
+              bool occ = pt.shadow_binary(sox, soy, soz, dxn, dyn, dzn, dist - 0.003f);
               float ws = occ ? 0.0f : ph * hsumWs / hph;
               float sum_s = cur_sumWs + ws, sum_u = cur_sumWu + wu;
               uint32_t newM = cur_M + hM; if (newM > uint32_t(mcap)) newM = uint32_t(mcap);
@@ -365,7 +367,7 @@ __global__ void __launch_bounds__(256, 3) k_restir_spatial(Scene s, Params p, ui
         if (!(ph_cur > 0.0f)) continue;
         float w_nbr_u = ph_cur * nbr_sumWu / nbr_ph;
         if (!(w_nbr_u > 0.0f)) continue;
-        bool occ = pt.occluded(sox, soy, soz, dxn, dyn, dzn, dist - 0.003f);
+        bool occ = pt.shadow_binary(sox, soy, soz, dxn, dyn, dzn, dist - 0.003f);
         float w_nbr_s = occ ? 0.0f : ph_cur * nbr_sumWs / nbr_ph;
         float sum_s = cur_sumWs + w_nbr_s, sum_u = cur_sumWu + w_nbr_u;
         if (!(sum_u > 0.0f) || !(sum_s >= 0.0f)) continue;

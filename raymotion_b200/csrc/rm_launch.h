@@ -210,6 +210,9 @@ struct DevBvh {
   int n_records = 0;
   int n_tris = 0;
   int max_depth = 0;
+  // 4-wide BVH collapsed from the records (rm_quad.cu): 8 float4 per node;
+  // qroots: nodes per level, then the binary record each node collapses
+  DevBuf quads, qroots;
   // 8-wide compressed BVH collapsed from the records (rm_wide.cu): 5 float4 per
   // node, triangle records in its leaf order, frontier queues; n_wide 0: none
   DevBuf wnodes, wtgeo, wq;
@@ -232,6 +235,10 @@ cudaError_t build_ploc(const rm_triangle* d_tris, int n_tris, int leaf_max, DevB
 cudaError_t pack_tgeo(const rm_triangle* d_tris, DevBvh& bvh, cudaStream_t st);
 // Refit all boxes bottom-up from the current triangle positions.
 cudaError_t refit_bvh(const rm_triangle* d_tris, DevBvh& bvh, cudaStream_t st);
+// Collapse the binary records (of a tree of depth max_depth) into the 4-wide
+// BVH, and copy their boxes into it after a refit (rm_quad.cu).
+cudaError_t build_quads(DevBvh& bvh, cudaStream_t st);
+cudaError_t refit_quads(DevBvh& bvh, cudaStream_t st);
 // Collapse the binary records into the 8-wide compressed BVH (rm_wide.cu).
 // Leaves n_wide at 0 (the binary BVH stays in use) when a node cannot be
 // encoded or the wide tree would be deeper than the traversal stack.

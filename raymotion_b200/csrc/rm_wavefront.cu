@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(256) k_wf_init(Scene s, Params p, uint64_t see
 
 // Traversal of a queue of rays, one thread per ray (closest hit for extension
 // rays, pathtrace.metal:119-163; any hit for shadow rays, :164).  T is the
-// traversal (Trav: binary BVH, WTrav: wide BVH) and E / kDepth its stack.
+// traversal (QTrav: 4-wide BVH, WTrav: 8-wide BVH) and E / kDepth its stack.
 // Finished extension rays are sorted into the shading queue of their surface
 // type.  (Persistent grids whose idle lanes claim new rays, per leaf-to-leaf
 // step or per node / triangle, measured 7-70 % slower on the 720p frame.)
@@ -494,7 +494,7 @@ __device__ __forceinline__ bool tail_step(const Scene& s, const Params& p, const
   if (ext) {
     const float4 o = w.o[id];
     const float4 d = w.d[id];
-    const TraceResult r = traverse<false>(s, o.x, o.y, o.z, d.x, d.y, d.z, kFar, err, cnt[1], cnt[2]);
+    const TraceResult r = traverse_quad<false>(s, o.x, o.y, o.z, d.x, d.y, d.z, kFar, err, cnt[1], cnt[2]);
     ++cnt[0];
     w.hit[id] = make_float4(r.t, r.u, r.v, __int_as_float(r.tri));
     if (r.tri >= 0) vk = __ldg(&s.tris[r.tri].ior) > 1.0001f ? 1 : 0;
@@ -502,7 +502,7 @@ __device__ __forceinline__ bool tail_step(const Scene& s, const Params& p, const
   if (w.u[id].y & kShadow) {
     const float4 o = w.so[id];
     const float4 d = w.sd[id];
-    const TraceResult r = traverse<true>(s, o.x, o.y, o.z, d.x, d.y, d.z, o.w, err, cnt[4], cnt[5]);
+    const TraceResult r = traverse_quad<true>(s, o.x, o.y, o.z, d.x, d.y, d.z, o.w, err, cnt[4], cnt[5]);
     ++cnt[3];
     w.occ[id] = r.tri >= 0 ? 1u : 0u;
   }
@@ -589,8 +589,8 @@ cudaError_t launch_wavefront_trace(const Scene& s, const WfState& w, const WfQue
     if (shadow) return trace_grid<true, WTrav, uint2, kWideStack>(s, w, q, bound, ctr, err, st);
     return trace_grid<false, WTrav, uint2, kWideStack>(s, w, q, bound, ctr, err, st);
   }
-  if (shadow) return trace_grid<true, Trav, int, kStack>(s, w, q, bound, ctr, err, st);
-  return trace_grid<false, Trav, int, kStack>(s, w, q, bound, ctr, err, st);
+  if (shadow) return trace_grid<true, QTrav, uint32_t, kQuadStack>(s, w, q, bound, ctr, err, st);
+  return trace_grid<false, QTrav, uint32_t, kQuadStack>(s, w, q, bound, ctr, err, st);
 }
 
 cudaError_t launch_wavefront_trace2(const Scene& s, const WfState& w, const WfQueues& q, int bound,

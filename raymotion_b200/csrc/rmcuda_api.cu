@@ -50,7 +50,12 @@ std::string cuda_msg(const char* what, cudaError_t e) { return std::string(what)
 
 namespace {
 
-constexpr int kLbvhLeaf = 4;
+// Triangles per leaf of the device-built BVHs.  Against four, leaves of two halve
+// the triangle tests for 6 % more node visits: plain frame 18.9 against 20.0
+// ms, a million closest-hit queries 461 against 481 us, the 720p ReSTIR frame
+// within its spread; of one, 17.4 ms and 482 us but the ReSTIR frame 118
+// against 113 ms.
+constexpr int kLbvhLeaf = 2;
 
 // The 8-wide compressed BVH, collapsed from the binary one (rm_wide.cu), when
 // RAYMOTION_CUDA_WIDE=1: traversal then uses it instead of the binary BVH.  It
@@ -64,7 +69,7 @@ cudaError_t finish_wide(rmd::DevBvh& bvh, cudaStream_t st) {
 }
 
 // Device BVH builder: PLOC clustering (default) or LBVH (RAYMOTION_CUDA_BVH=lbvh);
-// RAYMOTION_CUDA_BVH_LEAF sets the maximum triangles per leaf (default 4).
+// RAYMOTION_CUDA_BVH_LEAF sets the maximum triangles per leaf (default 2).
 cudaError_t build_device_bvh(const rm_triangle* d_tris, int n, rmd::DevBvh& bvh, cudaStream_t st, std::string& err) {
   int leaf = kLbvhLeaf;
   if (const char* v = std::getenv("RAYMOTION_CUDA_BVH_LEAF")) leaf = std::max(1, std::min(255, std::atoi(v)));
@@ -137,6 +142,7 @@ Scene scene_view(const DevScene& sc) {
   s.tgeo = sc.bvh.tgeo.as<float4>();
   s.nodes = sc.bvh.records.as<float4>();
   s.n_nodes = sc.n_tris > 0 ? sc.bvh.n_records : 0;
+  s.quads = sc.bvh.quads.as<float4>();
   s.lights = sc.lights.as<int32_t>();
   s.cdf = sc.cdf.as<float>();
   s.n_lights = sc.n_lights;
