@@ -144,22 +144,31 @@ __device__ __forceinline__ float unordered(unsigned int u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-__global__ void k_centroid_bounds(const rm_triangle* __restrict__ tris, int n, unsigned int* bounds) {
+// Six atomics per block: as one set per warp over a full grid, the atomics on
+// six words took 20 us whatever the size (1,000 triangles included).
+__global__ void __launch_bounds__(256) k_centroid_bounds(const rm_triangle* __restrict__ tris, int n,
+                                                         unsigned int* bounds) {
+  __shared__ unsigned int sh[6];
   unsigned int mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0, 0, 0};
+  if (threadIdx.x < 6) sh[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
+  __syncthreads();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const rm_triangle& t = tris[i];
     const float c[3] = {t.v0.x + t.v1.x + t.v2.x, t.v0.y + t.v1.y + t.v2.y, t.v0.z + t.v1.z + t.v2.z};
     for (int k = 0; k < 3; ++k) { mn[k] = min(mn[k], ordered(c[k])); mx[k] = max(mx[k], ordered(c[k])); }
   }
   for (int k = 0; k < 3; ++k) {
-    for (int o = 16; o; o >>= 1) {
-      mn[k] = min(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-      mx[k] = max(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-    }
+    mn[k] = __reduce_min_sync(0xffffffffu, mn[k]);
+    mx[k] = __reduce_max_sync(0xffffffffu, mx[k]);
   }
   if ((threadIdx.x & 31) == 0)
-    for (int k = 0; k < 3; ++k) { atomicMin(bounds + k, mn[k]); atomicMax(bounds + 3 + k, mx[k]); }
+    for (int k = 0; k < 3; ++k) { atomicMin(sh + k, mn[k]); atomicMax(sh + 3 + k, mx[k]); }
+  __syncthreads();
+  if (threadIdx.x < 3) atomicMin(bounds + threadIdx.x, sh[threadIdx.x]);
+  else if (threadIdx.x < 6) atomicMax(bounds + threadIdx.x, sh[threadIdx.x]);
 }
+
+static inline unsigned bounds_blocks(int n) { return unsigned(std::min(148 * 4, (n + 1023) / 1024)); }
 
 __device__ __forceinline__ unsigned int expand_bits(unsigned int v) {
   v = (v * 0x00010001u) & 0xFF0000FFu;
@@ -169,12 +178,8 @@ __device__ __forceinline__ unsigned int expand_bits(unsigned int v) {
   return v;
 }
 
-__global__ void k_morton(const rm_triangle* __restrict__ tris, int n, const unsigned int* __restrict__ bounds,
-                         unsigned int* __restrict__ keys, int* __restrict__ vals) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const rm_triangle& t = tris[i];
-  const float c[3] = {t.v0.x + t.v1.x + t.v2.x, t.v0.y + t.v1.y + t.v2.y, t.v0.z + t.v1.z + t.v2.z};
+// 30-bit Morton code of a centroid (times three) in the bounds.
+__device__ __forceinline__ unsigned int morton_code(const float* c, const unsigned int* bounds) {
   unsigned int q[3];
   for (int k = 0; k < 3; ++k) {
     const float lo = unordered(bounds[k]), hi = unordered(bounds[3 + k]);
@@ -183,7 +188,16 @@ __global__ void k_morton(const rm_triangle* __restrict__ tris, int n, const unsi
     f = fminf(fmaxf(f, 0.0f), 1.0f);
     q[k] = min(unsigned(f * 1024.0f), 1023u);
   }
-  keys[i] = (expand_bits(q[0]) << 2) | (expand_bits(q[1]) << 1) | expand_bits(q[2]);
+  return (expand_bits(q[0]) << 2) | (expand_bits(q[1]) << 1) | expand_bits(q[2]);
+}
+
+__global__ void k_morton(const rm_triangle* __restrict__ tris, int n, const unsigned int* __restrict__ bounds,
+                         unsigned int* __restrict__ keys, int* __restrict__ vals) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const rm_triangle& t = tris[i];
+  const float c[3] = {t.v0.x + t.v1.x + t.v2.x, t.v0.y + t.v1.y + t.v2.y, t.v0.z + t.v1.z + t.v2.z};
+  keys[i] = morton_code(c, bounds);
   vals[i] = i;
 }
 
@@ -196,11 +210,14 @@ __device__ __forceinline__ int delta(const unsigned int* keys, int n, int i, int
   return 32 + __clz(unsigned(i) ^ unsigned(j));
 }
 
-// Internal node i of n-1: children encoded as (index << 1) | is_leaf; ranges.
-__global__ void k_karras(const unsigned int* __restrict__ keys, int n, int2* __restrict__ children,
-                         int2* __restrict__ ranges, int* __restrict__ parent_int, int* __restrict__ parent_leaf) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n - 1) return;
+struct KarrasNode {
+  int left, right;  // child index
+  bool left_leaf, right_leaf;
+  int first, last;  // range of sorted positions
+};
+
+// Internal node i of n-1 (Karras 2012, algorithm 1); keys in global or shared memory.
+__device__ __forceinline__ KarrasNode karras_node(const unsigned int* keys, int n, int i) {
   const int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
   const int dmin = delta(keys, n, i, i - d);
   int lmax = 2;
@@ -216,13 +233,26 @@ __global__ void k_karras(const unsigned int* __restrict__ keys, int n, int2* __r
     if (t == 1) break;
   }
   const int gamma = i + s * d + min(d, 0);
-  const int first = min(i, j), last = max(i, j);
-  const int left = gamma, right = gamma + 1;
-  const bool left_leaf = (first == gamma), right_leaf = (last == gamma + 1);
-  children[i] = make_int2((left << 1) | int(left_leaf), (right << 1) | int(right_leaf));
-  ranges[i] = make_int2(first, last);
-  if (left_leaf) parent_leaf[left] = i; else parent_int[left] = i;
-  if (right_leaf) parent_leaf[right] = i; else parent_int[right] = i;
+  KarrasNode k;
+  k.first = min(i, j);
+  k.last = max(i, j);
+  k.left = gamma;
+  k.right = gamma + 1;
+  k.left_leaf = k.first == gamma;
+  k.right_leaf = k.last == gamma + 1;
+  return k;
+}
+
+// Children encoded as (index << 1) | is_leaf; ranges.
+__global__ void k_karras(const unsigned int* __restrict__ keys, int n, int2* __restrict__ children,
+                         int2* __restrict__ ranges, int* __restrict__ parent_int, int* __restrict__ parent_leaf) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n - 1) return;
+  const KarrasNode k = karras_node(keys, n, i);
+  children[i] = make_int2((k.left << 1) | int(k.left_leaf), (k.right << 1) | int(k.right_leaf));
+  ranges[i] = make_int2(k.first, k.last);
+  if (k.left_leaf) parent_leaf[k.left] = i; else parent_int[k.left] = i;
+  if (k.right_leaf) parent_leaf[k.right] = i; else parent_int[k.right] = i;
 }
 
 // Boxes of the Karras tree, bottom-up from the leaves; the sorted triangle
@@ -282,6 +312,173 @@ __global__ void k_emit_records(const rm_triangle* __restrict__ tris, const int* 
   rec[3] = make_float4(__int_as_float(links[0]), __int_as_float(links[1]), __int_as_float(counts[0]),
                        __int_as_float(counts[1]));
   if (i == 0) parents[0] = -1;
+}
+
+// The whole LBVH of a small scene in one block, for the no-allocation query,
+// whose cost at a thousand triangles was its launches: bounds, codes, sort, tree
+// and boxes ran as 17 kernels of 4 to 43 us (the boxes' climb, a fence and an
+// atomic in L2 per level, the longest).  Here the triangles are read once into
+// registers; the centroid bounds, the Morton codes, a bitonic sort of (code,
+// triangle) - the order the stable radix sort gives - and the keys stay in the
+// block (strides below a warp by shuffles); the boxes of every range of sorted
+// triangles come from a segment tree in shared memory, so that each internal
+// node finds its two children's boxes by itself, without a climb (the climb in
+// shared memory took 11 of 65 thousand cycles, the sort through shared memory
+// alone 19).  The records are those of the multi-kernel build.  4-wide nodes
+// instead (each node's internal children opened once, in the same pass)
+// traced 4,096 rays in 18.7 against 21.6 us and built in 30 against 25.
+constexpr int kSmallTris = 2048;
+
+struct SmallLbvh {
+  unsigned long long sorted[kSmallTris];  // code << 32 | triangle
+  unsigned int keys[kSmallTris];
+  int position[kSmallTris];   // sorted position of a triangle
+  Box tree[2 * kSmallTris];   // segment tree over the sorted triangles' boxes: leaf i at m + i
+  unsigned int bounds[6];
+};
+
+__device__ __forceinline__ unsigned long long shfl_xor_u64(unsigned long long v, int m) {
+  const unsigned lo = __shfl_xor_sync(0xffffffffu, unsigned(v), m);
+  const unsigned hi = __shfl_xor_sync(0xffffffffu, unsigned(v >> 32), m);
+  return ((unsigned long long)hi << 32) | lo;
+}
+
+// Box of the sorted positions [first, last] from a segment tree of m leaves.
+__device__ __forceinline__ Box range_box(const Box* tree, int m, int first, int last) {
+  Box b = empty_box();
+  for (int l = first + m, r = last + m + 1; l < r; l >>= 1, r >>= 1) {
+    if (l & 1) grow(b, tree[l++]);
+    if (r & 1) grow(b, tree[--r]);
+  }
+  return b;
+}
+
+__global__ void __launch_bounds__(1024) k_lbvh_small(const rm_triangle* __restrict__ tris, int n, int leaf_max,
+                                                     float4* __restrict__ recs, float4* __restrict__ tgeo,
+                                                     uint32_t* err_word) {
+  extern __shared__ __align__(16) unsigned char small_lbvh[];
+  SmallLbvh& sh = *reinterpret_cast<SmallLbvh*>(small_lbvh);
+  constexpr int kPer = kSmallTris / 1024;
+  const int tid = int(threadIdx.x);
+  if (tid == 0) *err_word = 0u;
+  if (tid < 6) sh.bounds[tid] = tid < 3 ? 0xffffffffu : 0u;
+  float v[kPer][9], c[kPer][3];
+  unsigned int mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0, 0, 0};
+  // the nine vertex floats of a 176-byte record: three 128-bit loads when the
+  // caller's array is aligned for them (the scalar loads of a warp touch 32
+  // lines nine times)
+  const bool wide = (reinterpret_cast<uintptr_t>(tris) & 15u) == 0;
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int j = tid + 1024 * r;
+    if (j >= n) continue;
+    const rm_triangle& t = tris[j];
+    if (wide) {
+      const float4* q = reinterpret_cast<const float4*>(&t);
+      const float4 a = q[0], b = q[1], d = q[2];
+      v[r][0] = a.x; v[r][1] = a.y; v[r][2] = a.z; v[r][3] = a.w;
+      v[r][4] = b.x; v[r][5] = b.y; v[r][6] = b.z; v[r][7] = b.w;
+      v[r][8] = d.x;
+    } else {
+      v[r][0] = t.v0.x; v[r][1] = t.v0.y; v[r][2] = t.v0.z;
+      v[r][3] = t.v1.x; v[r][4] = t.v1.y; v[r][5] = t.v1.z;
+      v[r][6] = t.v2.x; v[r][7] = t.v2.y; v[r][8] = t.v2.z;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      c[r][k] = v[r][k] + v[r][3 + k] + v[r][6 + k];
+      mn[k] = min(mn[k], ordered(c[r][k]));
+      mx[k] = max(mx[k], ordered(c[r][k]));
+    }
+  }
+  for (int k = 0; k < 3; ++k) {
+    mn[k] = __reduce_min_sync(0xffffffffu, mn[k]);
+    mx[k] = __reduce_max_sync(0xffffffffu, mx[k]);
+  }
+  __syncthreads();
+  if ((tid & 31) == 0 && tid < n)
+    for (int k = 0; k < 3; ++k) { atomicMin(sh.bounds + k, mn[k]); atomicMax(sh.bounds + 3 + k, mx[k]); }
+  __syncthreads();
+  int m = 32;
+  while (m < n) m <<= 1;
+  // element tid + 1024 r in e[r]
+  unsigned long long e[kPer];
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int j = tid + 1024 * r;
+    e[r] = j < n ? ((unsigned long long)(morton_code(c[r], sh.bounds)) << 32) | unsigned(j) : ~0ull;
+  }
+  for (int size = 2; size <= m; size <<= 1)
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      if (stride >= 1024) {  // both elements of a pair in this thread (size 2048: ascending)
+        if (e[0] > e[kPer - 1]) { const unsigned long long t = e[0]; e[0] = e[kPer - 1]; e[kPer - 1] = t; }
+        continue;
+      }
+      if (stride >= 32) {
+#pragma unroll
+        for (int r = 0; r < kPer; ++r)
+          if (tid + 1024 * r < m) sh.sorted[tid + 1024 * r] = e[r];
+        __syncthreads();
+      }
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) {
+        const int i = tid + 1024 * r;
+        const unsigned long long o =
+            stride >= 32 ? (i < m ? sh.sorted[i ^ stride] : ~0ull) : shfl_xor_u64(e[r], stride);
+        const bool low = (i & stride) == 0, up = (i & size) == 0;
+        if ((o < e[r]) == (low == up)) e[r] = o;
+      }
+      if (stride >= 32) __syncthreads();
+    }
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int i = tid + 1024 * r;
+    if (i < n) {
+      sh.keys[i] = unsigned(e[r] >> 32);
+      sh.position[unsigned(e[r])] = i;
+    } else if (i < m) {
+      sh.tree[m + i] = empty_box();
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kPer; ++r) {
+    const int j = tid + 1024 * r;
+    if (j >= n) continue;
+    const int pos = sh.position[j];
+    float4* g = tgeo + size_t(pos) * 3;
+    g[0] = make_float4(v[r][0], v[r][1], v[r][2], __int_as_float(j));
+    g[1] = make_float4(v[r][3] - v[r][0], v[r][4] - v[r][1], v[r][5] - v[r][2], 0.f);
+    g[2] = make_float4(v[r][6] - v[r][0], v[r][7] - v[r][1], v[r][8] - v[r][2], 0.f);
+    Box b;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      b.mn[k] = fminf(v[r][k], fminf(v[r][3 + k], v[r][6 + k]));
+      b.mx[k] = fmaxf(v[r][k], fmaxf(v[r][3 + k], v[r][6 + k]));
+    }
+    sh.tree[m + pos] = b;
+  }
+  __syncthreads();
+  for (int w = m >> 1; w >= 1; w >>= 1) {
+    for (int k = tid; k < w; k += 1024) {
+      Box b = sh.tree[2 * (w + k)];
+      grow(b, sh.tree[2 * (w + k) + 1]);
+      sh.tree[w + k] = b;
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < n - 1; i += 1024) {
+    const KarrasNode k = karras_node(sh.keys, n, i);
+    const int ln = k.left - k.first + 1, rn = k.last - k.right + 1;  // triangles of the children
+    const Box a = range_box(sh.tree, m, k.first, k.left), b = range_box(sh.tree, m, k.right, k.last);
+    const bool lleaf = ln <= leaf_max, rleaf = rn <= leaf_max;
+    float4* rec = recs + size_t(i) * 4;
+    rec[0] = make_float4(a.mn[0], a.mx[0], a.mn[1], a.mx[1]);
+    rec[1] = make_float4(b.mn[0], b.mx[0], b.mn[1], b.mx[1]);
+    rec[2] = make_float4(a.mn[2], a.mx[2], b.mn[2], b.mx[2]);
+    rec[3] = make_float4(__int_as_float(lleaf ? k.first : k.left), __int_as_float(k.right),
+                         __int_as_float(lleaf ? ln : 0), __int_as_float(rleaf ? rn : 0));
+  }
 }
 
 // Depth of each leaf slot (for the traversal stack bound).
@@ -455,7 +652,7 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(b.depth.reserve(sizeof(int)));
   unsigned int init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
   RM_TRY(cudaMemcpyAsync(b.bounds.ptr, init, sizeof(init), cudaMemcpyHostToDevice, st));
-  k_centroid_bounds<<<148 * 4, 256, 0, st>>>(d_tris, n, b.bounds.as<unsigned int>());
+  k_centroid_bounds<<<bounds_blocks(n), 256, 0, st>>>(d_tris, n, b.bounds.as<unsigned int>());
   unsigned int* keys = b.keys.as<unsigned int>();
   int* vals = reinterpret_cast<int*>(keys + n);
   k_morton<<<(n + 255) / 256, 256, 0, st>>>(d_tris, n, b.bounds.as<unsigned int>(), keys, vals);
@@ -496,11 +693,23 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
 cudaError_t build_lbvh_into(const rm_triangle* d_tris, int n, int leaf_max, const LbvhScratch& w, DevBvhView& out,
                             cudaStream_t st, std::string& err) {
   out.n_records = 0;
+  leaf_max = std::max(1, std::min(leaf_max, kMaxLeaf));
+  // One block up to kSmallTris triangles (above leaf_max), where the kernels of
+  // the large build are mostly launch: the call for 978 triangles and 4,096 rays took 213 us and
+  // takes 72, for 1,954 triangles 227 and 92.
+  if (n > leaf_max && n <= kSmallTris) {
+    RM_TRY(cudaFuncSetAttribute(k_lbvh_small, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SmallLbvh))));
+    k_lbvh_small<<<1, 1024, sizeof(SmallLbvh), st>>>(d_tris, n, leaf_max, w.records, w.tgeo, w.err_word);
+    RM_TRY(cudaGetLastError());
+    out.n_records = n - 1;
+    out.records = w.records;
+    out.tgeo = w.tgeo;
+    return cudaSuccess;
+  }
   // The error word lives in scratch shared by every call: clear it before any
   // early return, or an empty scene would report the last call's overflow.
   RM_TRY(cudaMemsetAsync(w.err_word, 0, sizeof(uint32_t), st));
   if (n <= 0) return cudaSuccess;
-  leaf_max = std::max(1, std::min(leaf_max, kMaxLeaf));
   if (n <= leaf_max) {
     k_single_leaf<<<1, 1, 0, st>>>(d_tris, n, w.records, w.parents, w.order);
     RM_TRY(cudaGetLastError());
@@ -510,7 +719,7 @@ cudaError_t build_lbvh_into(const rm_triangle* d_tris, int n, int leaf_max, cons
     // centroid bounds start at (+max ordered, 0): min slots all ones, max slots zero
     RM_TRY(cudaMemsetAsync(w.bounds, 0xff, 3 * sizeof(unsigned int), st));
     RM_TRY(cudaMemsetAsync(w.bounds + 3, 0, 3 * sizeof(unsigned int), st));
-    k_centroid_bounds<<<148 * 4, 256, 0, st>>>(d_tris, n, w.bounds);
+    k_centroid_bounds<<<bounds_blocks(n), 256, 0, st>>>(d_tris, n, w.bounds);
     k_morton<<<(n + 255) / 256, 256, 0, st>>>(d_tris, n, w.bounds, w.keys, w.vals);
     RM_TRY(cudaGetLastError());
     if (radix_sort_temp_bytes(n) > w.sort_temp_bytes) { err = "sort scratch too small"; return cudaErrorInvalidValue; }
@@ -563,9 +772,20 @@ __device__ __forceinline__ float half_area(const float4& lo, const float4& hi) {
   return dx * dy + dy * dz + dz * dx;
 }
 
+struct PlocState {
+  int clusters;   // current count
+  int next_node;  // id of the next node
+  int force;      // the last round merged nothing: merge neighbours (0,1), (2,3), ...
+  int side;       // which cluster list is current
+  // the round being applied
+  int in_clusters, in_force, in_side, in_next, merge;
+  unsigned int done;  // blocks of k_ploc_round that have counted
+};
+
 __global__ void k_ploc_leaves(const rm_triangle* __restrict__ tris, const int* __restrict__ order, int n,
-                              float4* __restrict__ blo, float4* __restrict__ bhi, int* __restrict__ cl) {
+                              float4* __restrict__ blo, float4* __restrict__ bhi, int* __restrict__ cl, PlocState* state) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *state = PlocState{n, n, 0, 0, 0, 0, 0, 0, 0, 0u};
   if (i >= n) return;
   const Box b = tri_box(tris[order[i]]);
   blo[i] = make_float4(b.mn[0], b.mn[1], b.mn[2], __int_as_float(1));
@@ -573,72 +793,275 @@ __global__ void k_ploc_leaves(const rm_triangle* __restrict__ tris, const int* _
   cl[i] = i;
 }
 
-__global__ void k_ploc_nn(const int* __restrict__ cl, int C, const float4* __restrict__ blo,
-                          const float4* __restrict__ bhi, int* __restrict__ nn) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= C) return;
-  const int a = cl[i];
-  const float4 alo = blo[a], ahi = bhi[a];
+// One round of the clustering is two launches, k_ploc_round and k_ploc_apply,
+// that read the cluster count on the device, so rounds are enqueued without
+// waiting for it; from kPlocSmall clusters on, one block runs the remaining
+// rounds (about half of them) in shared memory.  As nine launches and a
+// read-back a round, the 62 rounds of 400,000 triangles took
+// 2.7 ms of kernels and 62 waits; now 0.7 ms and one.
+constexpr int kPlocTile = 256;
+constexpr int kPlocSmall = 2048;
+
+// The nearest neighbour of cluster e of a staged window: lo / hi are the
+// window's boxes, w its length.
+__device__ __forceinline__ int ploc_nearest(const float4* lo, const float4* hi, int w, int e) {
+  const float4 alo = lo[e], ahi = hi[e];
   float best = __int_as_float(0x7f800000);
   int bj = -1;
-  const int j0 = max(0, i - kPlocRadius), j1 = min(C - 1, i + kPlocRadius);
+  const int j0 = max(0, e - kPlocRadius), j1 = min(w - 1, e + kPlocRadius);
   for (int j = j0; j <= j1; ++j) {
-    if (j == i) continue;
-    const int b = cl[j];
-    const float4 l = blo[b], h = bhi[b];
+    if (j == e) continue;
+    const float4 l = lo[j], h = hi[j];
     const float4 ulo = make_float4(fminf(alo.x, l.x), fminf(alo.y, l.y), fminf(alo.z, l.z), 0.f);
     const float4 uhi = make_float4(fmaxf(ahi.x, h.x), fmaxf(ahi.y, h.y), fmaxf(ahi.z, h.z), 0.f);
     const float area = half_area(ulo, uhi);
     if (area < best) { best = area; bj = j; }  // ties keep the smaller index (scanned in order)
   }
-  nn[i] = bj;
+  return bj;
 }
 
-// flags: x = this cluster creates a node, y = this cluster survives
-__global__ void k_ploc_flags(const int* __restrict__ nn, int C, int force, int* __restrict__ mflag,
-                             int* __restrict__ kflag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= C) return;
-  int j = nn[i];
-  bool mutual = j >= 0 && nn[j] == i;
-  if (force) {  // no mutual pair anywhere: merge neighbours (0,1), (2,3), ...
-    j = (i & 1) ? i - 1 : i + 1;
-    mutual = j < C;
+// The partner cluster i merges with, or -1; the smaller index creates the node.
+__device__ __forceinline__ int ploc_force_partner(int i, int C) {
+  const int j = (i & 1) ? i - 1 : i + 1;
+  return j < C ? j : -1;
+}
+
+// Per cluster: its mutual partner (pair[i], -1 for none); per block the nodes it
+// creates and the clusters that survive.  The boxes of a tile and of a halo of
+// two radii are staged in shared memory, so that the neighbours' own nearest
+// neighbours are found here as well.  The last block to finish scans the
+// blocks' counts and moves the state on.
+__global__ void __launch_bounds__(kPlocTile) k_ploc_round(const int* __restrict__ cl0, const int* __restrict__ cl1,
+                                                          const float4* __restrict__ blo,
+                                                          const float4* __restrict__ bhi, int* __restrict__ pair,
+                                                          int2* block_count, PlocState* st) {
+  constexpr int kHalo = 2 * kPlocRadius, kWin = kPlocTile + 2 * kHalo;
+  __shared__ float4 lo[kWin], hi[kWin];
+  __shared__ int near_[kPlocTile + 2 * kPlocRadius];
+  __shared__ int2 warp_sum[kPlocTile / 32];
+  __shared__ bool last;
+  const int C = st->clusters;
+  if (C <= kPlocSmall) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->merge = 0;  // nothing for k_ploc_apply
+    return;
   }
-  mflag[i] = (mutual && i < j) ? 1 : 0;
-  kflag[i] = (!mutual || i < j) ? 1 : 0;
+  const int blocks = (C + kPlocTile - 1) / kPlocTile;
+  if (int(blockIdx.x) >= blocks) return;
+  const int force = st->force;
+  const int* cl = st->side ? cl1 : cl0;
+  const int tile0 = int(blockIdx.x) * kPlocTile;
+  const int i = tile0 + int(threadIdx.x);
+  int partner = -1;
+  if (force) {
+    if (i < C) partner = ploc_force_partner(i, C);
+  } else {
+    const int w0 = max(0, tile0 - kHalo), w1 = min(C, tile0 + kPlocTile + kHalo);
+    for (int k = int(threadIdx.x); k < w1 - w0; k += kPlocTile) {
+      const int c = cl[w0 + k];
+      lo[k] = blo[c];
+      hi[k] = bhi[c];
+    }
+    __syncthreads();
+    const int n0 = max(0, tile0 - kPlocRadius), n1 = min(C, tile0 + kPlocTile + kPlocRadius);
+    for (int k = int(threadIdx.x); k < n1 - n0; k += kPlocTile)
+      near_[k] = w0 + ploc_nearest(lo, hi, w1 - w0, n0 + k - w0);
+    __syncthreads();
+    if (i < C) {
+      const int j = near_[i - n0];
+      if (j >= w0 && near_[j - n0] == i) partner = j;
+    }
+  }
+  if (i < C) pair[i] = partner;
+  const int creates = i < C && partner > i ? 1 : 0, stays = i < C && (partner < 0 || partner > i) ? 1 : 0;
+  const int2 c = make_int2(__reduce_add_sync(0xffffffffu, creates), __reduce_add_sync(0xffffffffu, stays));
+  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int2 t = make_int2(0, 0);
+    for (int w = 0; w < kPlocTile / 32; ++w) { t.x += warp_sum[w].x; t.y += warp_sum[w].y; }
+    block_count[blockIdx.x] = t;
+    __threadfence();
+    last = atomicAdd(&st->done, 1u) == unsigned(blocks) - 1u;
+  }
+  __syncthreads();
+  if (!last) return;
+  // exclusive scan of the blocks' counts, in place
+  __threadfence();
+  int2 carry = make_int2(0, 0);
+  for (int base = 0; base < blocks; base += kPlocTile) {
+    const int k = base + int(threadIdx.x);
+    int2 v = make_int2(0, 0);
+    if (k < blocks) {
+      v.x = __ldcg(&block_count[k].x);
+      v.y = __ldcg(&block_count[k].y);
+    }
+    int2 x = v;
+    const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int px = __shfl_up_sync(0xffffffffu, x.x, o), py = __shfl_up_sync(0xffffffffu, x.y, o);
+      if (lane >= o) { x.x += px; x.y += py; }
+    }
+    if (lane == 31) warp_sum[warp] = x;
+    __syncthreads();
+    int2 before = carry, all = make_int2(0, 0);
+    for (int w = 0; w < kPlocTile / 32; ++w) {
+      if (w < warp) { before.x += warp_sum[w].x; before.y += warp_sum[w].y; }
+      all.x += warp_sum[w].x;
+      all.y += warp_sum[w].y;
+    }
+    if (k < blocks) block_count[k] = make_int2(before.x + x.x - v.x, before.y + x.y - v.y);
+    carry.x += all.x;
+    carry.y += all.y;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    st->in_clusters = C;
+    st->in_force = force;
+    st->in_side = st->side;
+    st->in_next = st->next_node;
+    st->merge = carry.x > 0 ? 1 : 0;
+    st->done = 0u;
+    if (carry.x > 0) {
+      st->next_node += carry.x;
+      st->clusters = carry.y;
+      st->side ^= 1;
+      st->force = 0;
+    } else {
+      st->force = 1;  // degenerate input: pair up neighbours
+    }
+  }
 }
 
-__global__ void k_ploc_apply(const int* __restrict__ cl, const int* __restrict__ nn, int C, int force,
-                             const int* __restrict__ mflag, const int* __restrict__ mscan,
-                             const int* __restrict__ kflag, const int* __restrict__ kscan, int next_node,
-                             float4* __restrict__ blo, float4* __restrict__ bhi, int2* __restrict__ child,
-                             int* __restrict__ ncl, int n_leaves) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= C) return;
-  if (!kflag[i]) return;
+// A node of two clusters.
+__device__ __forceinline__ void ploc_merge(int a, int b, int id, int n_leaves, float4* blo, float4* bhi, int2* child,
+                                           float4& lo, float4& hi) {
+  const float4 al = blo[a], ah = bhi[a], bl = blo[b], bh = bhi[b];
+  const int size = __float_as_int(al.w) + __float_as_int(bl.w);
+  lo = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), __int_as_float(size));
+  hi = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), __int_as_float(-1));
+  blo[id] = lo;
+  bhi[id] = hi;
+  child[id - n_leaves] = make_int2(a, b);
+  bhi[a].w = __int_as_float(id);  // parent links
+  bhi[b].w = __int_as_float(id);
+}
+
+__global__ void __launch_bounds__(kPlocTile) k_ploc_apply(int* __restrict__ cl0, int* __restrict__ cl1,
+                                                          const int* __restrict__ pair,
+                                                          const int2* __restrict__ block_count, PlocState* st,
+                                                          float4* __restrict__ blo, float4* __restrict__ bhi,
+                                                          int2* __restrict__ child, int n_leaves) {
+  __shared__ int2 warp_sum[kPlocTile / 32];
+  const int C = st->in_clusters;
+  if (C <= kPlocSmall || !st->merge || int(blockIdx.x) * kPlocTile >= C) return;
+  const int* cl = st->in_side ? cl1 : cl0;
+  int* ncl = st->in_side ? cl0 : cl1;
+  const int i = int(blockIdx.x) * kPlocTile + int(threadIdx.x);
+  const int lane = int(threadIdx.x & 31), warp = int(threadIdx.x >> 5);
+  const int partner = i < C ? pair[i] : -1;
+  const bool creates = i < C && partner > i, stays = i < C && (partner < 0 || partner > i);
+  const unsigned cb = __ballot_sync(0xffffffffu, creates), sb = __ballot_sync(0xffffffffu, stays);
+  if (lane == 0) warp_sum[warp] = make_int2(__popc(cb), __popc(sb));
+  __syncthreads();
+  int2 pos = block_count[blockIdx.x];
+  for (int w = 0; w < warp; ++w) { pos.x += warp_sum[w].x; pos.y += warp_sum[w].y; }
+  pos.x += __popc(cb & ((1u << lane) - 1u));
+  pos.y += __popc(sb & ((1u << lane) - 1u));
+  if (!stays) return;
   int out = cl[i];
-  if (mflag[i]) {
-    const int j = force ? i + 1 : nn[i];
-    const int a = cl[i], b = cl[j];
-    const int id = next_node + mscan[i];
-    const float4 al = blo[a], ah = bhi[a], bl = blo[b], bh = bhi[b];
-    const int size = __float_as_int(al.w) + __float_as_int(bl.w);
-    blo[id] = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), __int_as_float(size));
-    bhi[id] = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), __int_as_float(-1));
-    child[id - n_leaves] = make_int2(a, b);
-    bhi[a].w = __int_as_float(id);  // parent links
-    bhi[b].w = __int_as_float(id);
+  if (creates) {
+    const int id = st->in_next + pos.x;
+    float4 lo, hi;
+    ploc_merge(out, cl[partner], id, n_leaves, blo, bhi, child, lo, hi);
     out = id;
   }
-  ncl[kscan[i]] = out;
+  ncl[pos.y] = out;
 }
 
-__global__ void k_ploc_totals(const int* __restrict__ mflag, const int* __restrict__ mscan,
-                              const int* __restrict__ kflag, const int* __restrict__ kscan, int C,
-                              int* __restrict__ totals) {
-  totals[0] = mscan[C - 1] + mflag[C - 1];
-  totals[1] = kscan[C - 1] + kflag[C - 1];
+// The rounds from kPlocSmall clusters to the root, one block.
+struct PlocSmall {
+  float4 lo[2][kPlocSmall], hi[2][kPlocSmall];
+  int id[2][kPlocSmall];
+  int near_[kPlocSmall];
+};
+
+__global__ void __launch_bounds__(1024) k_ploc_small(const int* __restrict__ cl0, const int* __restrict__ cl1,
+                                                     PlocState* st, float4* __restrict__ blo,
+                                                     float4* __restrict__ bhi, int2* __restrict__ child,
+                                                     int n_leaves) {
+  extern __shared__ __align__(16) unsigned char ploc_small[];
+  PlocSmall& sh = *reinterpret_cast<PlocSmall*>(ploc_small);
+  __shared__ int2 warp_sum[32];
+  const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
+  int C = st->clusters, next = st->next_node;
+  bool force = st->force != 0;
+  if (C > kPlocSmall) return;  // not reached yet
+  const int* cl = st->side ? cl1 : cl0;
+  for (int i = tid; i < C; i += 1024) {
+    const int c = cl[i];
+    sh.id[0][i] = c;
+    sh.lo[0][i] = blo[c];
+    sh.hi[0][i] = bhi[c];
+  }
+  __syncthreads();
+  int cur = 0;
+  for (int round = 0; C > 1 && round < 2 * kPlocSmall; ++round) {  // a round merges, or the next one does
+    if (!force)
+      for (int i = tid; i < C; i += 1024) sh.near_[i] = ploc_nearest(sh.lo[cur], sh.hi[cur], C, i);
+    __syncthreads();
+    int2 carry = make_int2(0, 0);
+    for (int base = 0; base < C; base += 1024) {
+      const int i = base + tid;
+      int partner = -1;
+      if (i < C) {
+        if (force) partner = ploc_force_partner(i, C);
+        else {
+          const int j = sh.near_[i];
+          if (j >= 0 && sh.near_[j] == i) partner = j;
+        }
+      }
+      const bool creates = i < C && partner > i, stays = i < C && (partner < 0 || partner > i);
+      const unsigned cb = __ballot_sync(0xffffffffu, creates), sb = __ballot_sync(0xffffffffu, stays);
+      if (lane == 0) warp_sum[warp] = make_int2(__popc(cb), __popc(sb));
+      __syncthreads();
+      int2 pos = carry;
+      for (int w = 0; w < 32; ++w) {
+        const int2 q = warp_sum[w];
+        if (w < warp) { pos.x += q.x; pos.y += q.y; }
+        carry.x += q.x;
+        carry.y += q.y;
+      }
+      pos.x += __popc(cb & ((1u << lane) - 1u));
+      pos.y += __popc(sb & ((1u << lane) - 1u));
+      if (stays) {
+        const int o = cur ^ 1;
+        sh.id[o][pos.y] = sh.id[cur][i];
+        sh.lo[o][pos.y] = sh.lo[cur][i];
+        sh.hi[o][pos.y] = sh.hi[cur][i];
+        if (creates) {
+          const int id = next + pos.x;
+          float4 lo, hi;
+          ploc_merge(sh.id[cur][i], sh.id[cur][partner], id, n_leaves, blo, bhi, child, lo, hi);
+          sh.id[o][pos.y] = id;
+          sh.lo[o][pos.y] = lo;
+          sh.hi[o][pos.y] = hi;
+        }
+      }
+      __syncthreads();
+    }
+    force = carry.x == 0;
+    if (carry.x > 0) {
+      next += carry.x;
+      C = carry.y;
+      cur ^= 1;
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    st->clusters = C;
+    st->next_node = next;
+  }
 }
 
 // Leaf position in depth-first order and depth: walk to the root adding the
@@ -651,6 +1074,7 @@ __global__ void k_ploc_layout(int n, int root, const float4* __restrict__ blo, c
   int off = 0, d = 1, cur = i;
   while (cur != root) {
     const int p = __float_as_int(bhi[cur].w);
+    if (p < n) break;  // no parent: an unfinished tree
     const int2 c = child[p - n];
     if (c.y == cur) off += __float_as_int(blo[c.x].w);
     cur = p;
@@ -673,6 +1097,7 @@ __global__ void k_ploc_preorder(int n, int root, const float4* __restrict__ blo,
   int off = 0, d = 0, cur = n + k;
   while (cur != root) {
     const int p = __float_as_int(bhi[cur].w);
+    if (p < n) break;  // no parent: an unfinished tree
     const int2 c = child[p - n];
     off += 1;
     if (c.y == cur) off += __float_as_int(blo[c.x].w) - 1;
@@ -746,7 +1171,7 @@ cudaError_t build_ploc(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(b.vals_alt.reserve(size_t(n) * 4));
   unsigned int init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
   RM_TRY(cudaMemcpyAsync(b.bounds.ptr, init, sizeof(init), cudaMemcpyHostToDevice, st));
-  k_centroid_bounds<<<148 * 4, 256, 0, st>>>(d_tris, n, b.bounds.as<unsigned int>());
+  k_centroid_bounds<<<bounds_blocks(n), 256, 0, st>>>(d_tris, n, b.bounds.as<unsigned int>());
   unsigned int* keys = b.keys.as<unsigned int>();
   int* vals = reinterpret_cast<int*>(keys + n);
   k_morton<<<(n + 255) / 256, 256, 0, st>>>(d_tris, n, b.bounds.as<unsigned int>(), keys, vals);
@@ -757,58 +1182,50 @@ cudaError_t build_ploc(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(radix_sort_pairs(keys, b.keys_alt.as<unsigned int>(), vals, b.vals_alt.as<int>(), n, 30, b.temp.ptr,
                           sort_bytes, in_alt, st));
   const int* sorted = in_alt ? b.vals_alt.as<int>() : vals;
-  // node and cluster arrays (kbox: box lo/hi; knodes: children; ranges: 2 cluster lists + nn + 4 flag arrays)
+  // node and cluster arrays (kbox: box lo/hi; knodes: children; ranges: two cluster lists, pairs, block counts, state)
+  const int tiles = (n + kPlocTile - 1) / kPlocTile;
   RM_TRY(b.kbox.reserve(size_t(total) * 2 * sizeof(float4)));
   RM_TRY(b.knodes.reserve(size_t(n) * sizeof(int2)));
-  RM_TRY(b.ranges.reserve(size_t(n) * 7 * sizeof(int) + 2 * sizeof(int)));
+  RM_TRY(b.ranges.reserve(size_t(n) * 3 * sizeof(int) + sizeof(int) + size_t(tiles) * sizeof(int2) + sizeof(PlocState)));
   RM_TRY(b.kcount.reserve(size_t(n) * sizeof(int)));
+  RM_TRY(b.depth.reserve(sizeof(int)));
   float4* blo = b.kbox.as<float4>();
   float4* bhi = blo + total;
   int2* child = b.knodes.as<int2>();
-  int* cl0 = b.ranges.as<int>();
+  int2* block_count = b.ranges.as<int2>();
+  PlocState* state = reinterpret_cast<PlocState*>(block_count + tiles);
+  int* cl0 = reinterpret_cast<int*>(state + 1);
   int* cl1 = cl0 + n;
-  int* nn = cl1 + n;
-  int* mflag = nn + n;
-  int* mscan = mflag + n;
-  int* kflag = mscan + n;
-  int* kscan = kflag + n;
-  int* totals = kscan + n;
-  k_ploc_leaves<<<(n + 255) / 256, 256, 0, st>>>(d_tris, sorted, n, blo, bhi, cl0);
+  int* pair = cl1 + n;
+  k_ploc_leaves<<<(n + 255) / 256, 256, 0, st>>>(d_tris, sorted, n, blo, bhi, cl0, state);
   RM_TRY(cudaGetLastError());
-  int C = n, next_node = n, iters = 0;
-  int* cl = cl0;
-  int* ncl = cl1;
-  int h_tot[2];
-  while (C > 1) {
-    if (++iters > 4 * n + 64) { err = "clustering build did not converge"; return cudaErrorInvalidValue; }
-    const unsigned g = unsigned((C + 255) / 256);
-    int force = 0;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      if (!force) k_ploc_nn<<<g, 256, 0, st>>>(cl, C, blo, bhi, nn);
-      k_ploc_flags<<<g, 256, 0, st>>>(nn, C, force, mflag, kflag);
-      RM_TRY(exclusive_scan(mflag, mscan, C, b.temp.ptr, scan_bytes, st));
-      RM_TRY(exclusive_scan(kflag, kscan, C, b.temp.ptr, scan_bytes, st));
-      k_ploc_totals<<<1, 1, 0, st>>>(mflag, mscan, kflag, kscan, C, totals);
-      RM_TRY(cudaMemcpyAsync(h_tot, totals, sizeof(h_tot), cudaMemcpyDeviceToHost, st));
-      RM_TRY(cudaStreamSynchronize(st));
-      if (h_tot[0] > 0) break;
-      force = 1;  // degenerate input: pair up neighbours
+  RM_TRY(cudaFuncSetAttribute(k_ploc_small, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(PlocSmall))));
+  // Rounds in batches: a round keeps about two thirds of the clusters, so the
+  // first batch usually ends below kPlocSmall; the count read back after it
+  // says whether more are needed (launches past the end return at once).
+  long long rounds = 0;
+  for (int C = n; C > kPlocSmall;) {
+    const unsigned g = unsigned((C + kPlocTile - 1) / kPlocTile);
+    int batch = 2;
+    for (double c = C; c > kPlocSmall; c *= 0.66) ++batch;
+    for (int k = 0; k < batch; ++k) {
+      k_ploc_round<<<g, kPlocTile, 0, st>>>(cl0, cl1, blo, bhi, pair, block_count, state);
+      k_ploc_apply<<<g, kPlocTile, 0, st>>>(cl0, cl1, pair, block_count, state, blo, bhi, child, n);
     }
-    k_ploc_apply<<<g, 256, 0, st>>>(cl, nn, C, force, mflag, mscan, kflag, kscan, next_node, blo, bhi, child, ncl, n);
     RM_TRY(cudaGetLastError());
-    next_node += h_tot[0];
-    C = h_tot[1];
-    std::swap(cl, ncl);
+    if ((rounds += batch) > 8ll * n + 64) { err = "clustering build did not converge"; return cudaErrorInvalidValue; }
+    RM_TRY(cudaMemcpyAsync(&C, &state->clusters, sizeof(int), cudaMemcpyDeviceToHost, st));
+    RM_TRY(cudaStreamSynchronize(st));
   }
-  const int root = next_node - 1;
-  if (root != total - 1) { err = "clustering build produced a malformed tree"; return cudaErrorInvalidValue; }
-  // layout
+  k_ploc_small<<<1, 1024, sizeof(PlocSmall), st>>>(cl0, cl1, state, blo, bhi, child, n);
+  RM_TRY(cudaGetLastError());
+  const int root = total - 1;
+  // layout (of a complete tree: an unfinished one, whose root is missing, ends the walks at their bound)
   int* pos = b.kcount.as<int>();
-  RM_TRY(b.depth.reserve(sizeof(int)));
   RM_TRY(cudaMemsetAsync(b.depth.ptr, 0, sizeof(int), st));
   k_ploc_layout<<<(n + 255) / 256, 256, 0, st>>>(n, root, blo, bhi, child, sorted, pos, b.order.as<int>(),
                                                  b.depth.as<int>());
-  int* pre = nn;  // the cluster arrays are free once the tree is built
+  int* pre = pair;  // the cluster arrays are free once the tree is built
   k_ploc_preorder<<<(n - 1 + 255) / 256, 256, 0, st>>>(n, root, blo, bhi, child, pre);
   RM_TRY(b.records.reserve(size_t(n - 1) * 4 * sizeof(float4)));
   RM_TRY(b.parents.reserve(size_t(n - 1) * sizeof(int)));

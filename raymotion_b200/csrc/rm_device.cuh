@@ -670,6 +670,18 @@ __device__ __forceinline__ TraceResult traverse_rt(const Scene& s, float ox, flo
   return t.r;
 }
 
+// traverse_quad() with the any-hit rule as a run-time flag.
+__device__ __forceinline__ TraceResult traverse_quad_rt(const Scene& s, float ox, float oy, float oz, float dx,
+                                                        float dy, float dz, float tmax, bool any_hit, uint32_t* err,
+                                                        uint32_t& n_nodes, uint32_t& n_tests) {
+  QTrav t;
+  uint32_t stack[kQuadStack];
+  t.init(ox, oy, oz, dx, dy, dz, tmax);
+  while (!t.step_rt(s, stack, err, n_nodes, n_tests, any_hit)) {
+  }
+  return t.r;
+}
+
 // One ray through the binary records (Trav).
 template <bool kAnyHit>
 __device__ __forceinline__ TraceResult traverse(const Scene& s, float ox, float oy, float oz, float dx, float dy,
@@ -690,8 +702,6 @@ template <bool kAnyHit>
 __device__ __forceinline__ TraceResult traverse_any(const Scene& s, float ox, float oy, float oz, float dx, float dy,
                                                     float dz, float tmax, uint32_t* err, uint32_t& n_nodes,
                                                     uint32_t& n_tests) {
-  // the no-allocation query builds only the binary records
-  if (!s.quads) return traverse<kAnyHit>(s, ox, oy, oz, dx, dy, dz, tmax, err, n_nodes, n_tests);
   if (s.wnodes) {
     WTrav t;
     uint2 stack[kWideStack];

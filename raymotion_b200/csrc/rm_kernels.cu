@@ -11,6 +11,8 @@
 
 namespace rmd {
 
+constexpr int kQueryThreads = 64;
+
 // Warp-aggregated counter update; every lane of the warp must reach it.
 __device__ __forceinline__ void warp_count(unsigned long long* ctr, uint32_t v) {
   unsigned long long s = __reduce_add_sync(0xffffffffu, v);
@@ -639,15 +641,23 @@ __global__ void __launch_bounds__(256) k_restir_shade(Scene s, Params p, uint64_
   flush_counts(ctr, taken, rays, nodes, tests);
 }
 
-// Closest-hit / any-hit query kernel behind rmcuda_trace.
-__global__ void __launch_bounds__(256) k_trace(Scene s, const float* __restrict__ rays, int n, int any_hit,
-                                               int32_t* __restrict__ tri, float* t, float* u, float* v, uint32_t* err) {
+// Closest-hit / any-hit query kernel behind rmcuda_trace and
+// rmcuda_trace_noalloc: WIDTH 2 (the no-allocation query builds only the binary
+// records), 4, or 8 when the scene has that BVH.
+template <int WIDTH>
+__global__ void __launch_bounds__(kQueryThreads) k_trace(Scene s, const float* __restrict__ rays, int n, int any_hit,
+                                                         int32_t* __restrict__ tri, float* t, float* u, float* v,
+                                                         uint32_t* err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* r = rays + size_t(i) * 7;
   uint32_t nodes = 0, tests = 0;
-  TraceResult h = any_hit ? traverse_any<true>(s, r[0], r[1], r[2], r[3], r[4], r[5], r[6], err, nodes, tests)
-                          : traverse_any<false>(s, r[0], r[1], r[2], r[3], r[4], r[5], r[6], err, nodes, tests);
+  const bool any = any_hit != 0;
+  TraceResult h;
+  if (WIDTH == 2) h = traverse_rt(s, r[0], r[1], r[2], r[3], r[4], r[5], r[6], any, err, nodes, tests);
+  else if (WIDTH == 4) h = traverse_quad_rt(s, r[0], r[1], r[2], r[3], r[4], r[5], r[6], any, err, nodes, tests);
+  else h = any ? traverse_any<true>(s, r[0], r[1], r[2], r[3], r[4], r[5], r[6], err, nodes, tests)
+               : traverse_any<false>(s, r[0], r[1], r[2], r[3], r[4], r[5], r[6], err, nodes, tests);
   tri[i] = h.tri;
   if (t) t[i] = h.tri >= 0 ? h.t : r[6];
   if (u) u[i] = h.u;
@@ -682,7 +692,10 @@ cudaError_t launch_restir_stage(int stage, const Scene& s, const Params& p, uint
 cudaError_t launch_trace(const Scene& s, const float* rays, int n, int any_hit, int32_t* tri, float* t, float* u,
                          float* v, uint32_t* err, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  k_trace<<<blocks_for(uint64_t(n), 256), 256, 0, st>>>(s, rays, n, any_hit, tri, t, u, v, err);
+  const unsigned g = blocks_for(uint64_t(n), kQueryThreads);
+  if (s.wnodes) k_trace<8><<<g, kQueryThreads, 0, st>>>(s, rays, n, any_hit, tri, t, u, v, err);
+  else if (s.quads) k_trace<4><<<g, kQueryThreads, 0, st>>>(s, rays, n, any_hit, tri, t, u, v, err);
+  else k_trace<2><<<g, kQueryThreads, 0, st>>>(s, rays, n, any_hit, tri, t, u, v, err);
   return cudaGetLastError();
 }
 
