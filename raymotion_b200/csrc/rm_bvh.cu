@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "rm_launch.h"
@@ -34,19 +35,98 @@ namespace rmd {
   } while (0)
 
 
+namespace {
+
+constexpr int kPoolDevices = 64;
+struct DevicePool {
+  std::mutex mu;
+  int users = 0;
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t stream = nullptr;  // orders the pool's own allocations and frees; carries no work
+};
+DevicePool g_pools[kPoolDevices];
+
+}  // namespace
+
+void pool_open(int device) {
+  if (device < 0 || device >= kPoolDevices) return;
+  DevicePool& p = g_pools[device];
+  std::lock_guard<std::mutex> lk(p.mu);
+  if (p.users++ > 0) return;
+  int supported = 0;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  unsigned long long keep = kPoolKeep;
+  if (cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && supported &&
+      cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) == cudaSuccess &&
+      cudaMemPoolCreate(&p.pool, &props) == cudaSuccess &&
+      cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+    return;
+  // no pool here: cudaMalloc serves the buffers
+  cudaGetLastError();
+  if (p.pool) cudaMemPoolDestroy(p.pool);
+  if (p.stream) cudaStreamDestroy(p.stream);
+  p.pool = nullptr;
+  p.stream = nullptr;
+}
+
+void pool_close(int device) {
+  if (device < 0 || device >= kPoolDevices) return;
+  DevicePool& p = g_pools[device];
+  std::lock_guard<std::mutex> lk(p.mu);
+  if (--p.users > 0) return;
+  if (p.stream) cudaStreamSynchronize(p.stream);
+  if (p.pool) cudaMemPoolDestroy(p.pool);
+  if (p.stream) cudaStreamDestroy(p.stream);
+  p.pool = nullptr;
+  p.stream = nullptr;
+}
+
 cudaError_t DevBuf::reserve(size_t bytes) {
   if (bytes <= cap && ptr) return cudaSuccess;
-  if (ptr) { cudaFree(ptr); ptr = nullptr; cap = 0; }
-  size_t want = std::max<size_t>(bytes, 256);
+  if (ptr) release();
+  const size_t want = std::max<size_t>(bytes, 256);
+  int dev = -1;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kPoolDevices) {
+    DevicePool& p = g_pools[dev];
+    std::lock_guard<std::mutex> lk(p.mu);
+    if (p.pool) {
+      // complete before any other stream can be given the pointer
+      cudaError_t e = cudaMallocFromPoolAsync(&ptr, want, p.pool, p.stream);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(p.stream);
+      if (e != cudaSuccess) { ptr = nullptr; return e; }
+      cap = want;
+      device = dev;
+      return cudaSuccess;
+    }
+  }
   cudaError_t e = cudaMalloc(&ptr, want);
   if (e != cudaSuccess) { ptr = nullptr; return e; }
   cap = want;
+  device = -1;
   return cudaSuccess;
 }
+
 void DevBuf::release() {
-  if (ptr) cudaFree(ptr);
+  if (ptr && device >= 0) {
+    int now = device;
+    cudaGetDevice(&now);
+    if (now != device) cudaSetDevice(device);
+    // any stream of any context may still use the memory: wait, as cudaFree does
+    cudaDeviceSynchronize();
+    DevicePool& p = g_pools[device];
+    std::lock_guard<std::mutex> lk(p.mu);
+    if (p.pool) cudaFreeAsync(ptr, p.stream);
+    else cudaFree(ptr);  // the pool went with its last context; its memory goes back here
+    if (now != device) cudaSetDevice(now);
+  } else if (ptr) {
+    cudaFree(ptr);
+  }
   ptr = nullptr;
   cap = 0;
+  device = -1;
 }
 
 namespace {
@@ -524,6 +604,22 @@ __global__ void k_differ(const uint4* __restrict__ a, const uint4* __restrict__ 
   if (__any_sync(0xffffffffu, d) && (threadIdx.x & 31) == 0) atomicOr(flag, 1);
 }
 
+// What upload_scene asks of every triangle before it is used (see check_triangles).
+__global__ void __launch_bounds__(256) k_check_triangles(const rm_triangle* __restrict__ tris, int n,
+                                                         long long n_texels, int* flags) {
+  int f = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const rm_triangle& t = tris[i];
+    if (!(t.alpha >= 1.0f)) f |= 1;
+    if (t.texture_offset >= 0 &&
+        (t.texture_width <= 0 || t.texture_height <= 0 ||
+         (long long)t.texture_offset + (long long)t.texture_width * t.texture_height > n_texels))
+      f |= 2;
+  }
+  f = __reduce_or_sync(0xffffffffu, f);
+  if ((threadIdx.x & 31) == 0 && f) atomicOr(flags, f);
+}
+
 __global__ void k_light_records(const rm_triangle* __restrict__ tris, const int32_t* __restrict__ lights, int n,
                                 float4* __restrict__ rec) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -594,6 +690,13 @@ cudaError_t refit_bvh(const rm_triangle* d_tris, DevBvh& bvh, cudaStream_t st) {
   if (e == cudaSuccess) e = refit_quads(bvh, st);
   if (e != cudaSuccess) return e;
   return pack_tgeo(d_tris, bvh, st);
+}
+
+cudaError_t check_triangles(const rm_triangle* d_tris, int n, long long n_texels, int* d_flags, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(d_flags, 0, sizeof(int), st);
+  if (e != cudaSuccess || n <= 0) return e;
+  k_check_triangles<<<unsigned(std::min(148 * 4, (n + 255) / 256)), 256, 0, st>>>(d_tris, n, n_texels, d_flags);
+  return cudaGetLastError();
 }
 
 cudaError_t device_differ(const void* a, const void* b, size_t n_bytes, int* d_flag, cudaStream_t st) {

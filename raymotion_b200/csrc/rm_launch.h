@@ -189,11 +189,23 @@ cudaError_t launch_atrous_tiled(int step, const Params& p, const GBufSoA& gb, co
 
 // rm_bvh.cu ------------------------------------------------------------------
 
-// Growable device allocation.
+// Device memory of the contexts on one device: a stream-ordered pool, made by
+// the device's first context and destroyed with its last (pool_open /
+// pool_close, one pair per context).  A cudaMalloc or cudaFree takes 0.25 to
+// 0.5 ms, and a scene needs about 28 buffers, a context's first ReSTIR frame
+// about 70; memory that a scene or a context gave back serves the next from
+// the pool in microseconds.  At most kPoolKeep bytes stay in it unused.
+constexpr unsigned long long kPoolKeep = 2ull << 30;
+void pool_open(int device);
+void pool_close(int device);
+
+// Growable device allocation on the device that was current at reserve().
 struct DevBuf {
   void* ptr = nullptr;
   size_t cap = 0;
+  int device = -1;  // >= 0: from that device's pool
   cudaError_t reserve(size_t bytes);
+  // waits for the device, as cudaFree does, and gives the memory back
   void release();
   template <class T> T* as() const { return static_cast<T*>(ptr); }
 };
@@ -278,6 +290,9 @@ size_t lbvh_box_bytes();
 cudaError_t prepare_lights(const rm_triangle* d_tris, const int32_t* d_lights, const float* d_cdf, int n_lights,
                            float light_total, DevBuf& rec, DevBuf& guide, int& guide_n, float& guide_inv,
                            cudaStream_t st);
+// d_flags[0]: bit 0 when a triangle is not opaque, bit 1 when one's texture
+// lies outside the n_texels texels.
+cudaError_t check_triangles(const rm_triangle* d_tris, int n, long long n_texels, int* d_flags, cudaStream_t st);
 // d_flag[0] = 1 when the two device byte ranges differ, else 0 (n_bytes a multiple of 16).
 cudaError_t device_differ(const void* a, const void* b, size_t n_bytes, int* d_flag, cudaStream_t st);
 // 64-bit content hash of a device byte range (order-sensitive per 8-byte word).
