@@ -33,7 +33,7 @@ NVFLAGS = ARCH + [
     "-prec-div=true", "-prec-sqrt=true", "-ftz=false",
     f"-I{ROOT / 'include'}", f"-I{CSRC}",
 ]
-CU_SOURCES = ["rm_kernels.cu", "rm_denoise.cu", "rm_bvh.cu", "rmcuda_api.cu", "rm_noalloc.cu", "rm_wavefront.cu",
+CU_SOURCES = ["rm_kernels.cu", "rm_paths.cu", "rm_denoise.cu", "rm_bvh.cu", "rmcuda_api.cu", "rm_noalloc.cu", "rm_wavefront.cu",
               "rm_atrous.cu", "rm_batch.cu", "rmcuda_batch.cu", "rm_adjoint.cu", "rm_denoise_adjoint.cu",
               "rmcuda_adjoint.cu", "rm_wide.cu", "rm_quad.cu", "rm_prep.cu", "rm_sort.cu"]
 # Tolerance-checked kernels (approximate exp2 / rsqrt anyway) are compiled with FMA contraction.

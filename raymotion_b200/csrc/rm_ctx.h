@@ -133,6 +133,8 @@ struct rmcuda_ctx {
   rmapi::ResSet rinit, rmerged, hres;
   rmd::DevBuf hdr, tmp_a, tmp_b, hist_col, rgb, dbg, hash_out;
   rmd::DevBuf ctr, err;
+  rmd::DevBuf paths;  // values, states, sums and lists of a plain frame (rm_paths.cu)
+  int sms = 0;
   // speculative frames of rmcuda_render: the copy stream that uploads and
   // compares the triangles while the frame renders, its pinned result, a copy
   // of the counters to restore, and the configuration of the last frame

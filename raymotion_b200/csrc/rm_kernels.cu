@@ -35,10 +35,10 @@ __device__ __forceinline__ void clamp3(const Params& p, float& r, float& g, floa
   }
 }
 
-// K1 render_paths (pathtrace.metal:739-769) for LANES == 1, and K2
-// render_paths_simd (:773-815) for LANES in {8, 32}: LANES threads per pixel,
-// each a strided subset of the samples, reduced with butterfly shuffles that
-// never leave the pixel's lane group.
+// K2 render_paths_simd (pathtrace.metal:773-815) in one launch, for small
+// frames with adaptive sampling (the others: rm_paths.cu): LANES (8 or 32)
+// threads per pixel, each a strided subset of the samples, reduced with
+// butterfly shuffles that never leave the pixel's lane group.
 template <int LANES>
 __global__ void __launch_bounds__(256) k_render_paths(Scene s, Params p, uint64_t seed, float* __restrict__ hdr,
                                                       uint8_t* __restrict__ rgb, uint32_t* __restrict__ dbg,
@@ -51,69 +51,43 @@ __global__ void __launch_bounds__(256) k_render_paths(Scene s, Params p, uint64_
     const uint32_t x = pixel % uint32_t(p.width), y = pixel / uint32_t(p.width);
     Tracer pt(s, p, err);
     uint64_t sd = seed_pixel(seed, x, y);
-    if (LANES > 1) sd ^= uint64_t(lane) * 0x94D049BB133111EBull;
+    sd ^= uint64_t(lane) * 0x94D049BB133111EBull;
     pt.rng.seed(sd);
     float sr = 0, sg = 0, sb = 0, sum_l = 0, sum_l2 = 0;
     int n = 0;
-    if (LANES == 1) {
-      for (int si = 0; si < p.spp; ++si) {
-        float sx, sy, cr, cg, cb;
+    const uint32_t group = (threadIdx.x & 31u) / LANES;
+    const uint32_t mask = LANES == 32 ? 0xffffffffu : (((1u << LANES) - 1u) << (group * LANES));
+    for (uint32_t base = 0; base < uint32_t(p.spp); base += LANES) {
+      float cr = 0, cg = 0, cb = 0;
+      if (base + lane < uint32_t(p.spp)) {
+        float sx, sy;
         pt.jitter(x, y, sx, sy);
         pt.sample_sensor(sx, sy, p.bounces, cr, cg, cb);
         clamp3(p, cr, cg, cb);
-        sr += cr; sg += cg; sb += cb;
-        ++n;
-        if (p.adapt_min > 0) {
-          float lum = cr * 0.2126f + cg * 0.7152f + cb * 0.0722f;
-          sum_l += lum; sum_l2 += lum * lum;
-          if (n >= p.adapt_min && n > 1 && n % p.adapt_step == 0) {
-            float mean = sum_l / float(n);
-            float var = fmaxf(0.0f, (sum_l2 - sum_l * mean) / float(n - 1));
-            float thr = p.adapt_rel * mean + p.adapt_abs;
-            if (var < thr * thr) break;
-          }
-        }
+        ++taken;
       }
-      taken = uint32_t(n);
-    } else {
-      const uint32_t group = (threadIdx.x & 31u) / LANES;
-      const uint32_t mask = LANES == 32 ? 0xffffffffu : (((1u << LANES) - 1u) << (group * LANES));
-      for (uint32_t base = 0; base < uint32_t(p.spp); base += LANES) {
-        float cr = 0, cg = 0, cb = 0;
-        if (base + lane < uint32_t(p.spp)) {
-          float sx, sy;
-          pt.jitter(x, y, sx, sy);
-          pt.sample_sensor(sx, sy, p.bounces, cr, cg, cb);
-          clamp3(p, cr, cg, cb);
-          ++taken;
-        }
-        float lum = cr * 0.2126f + cg * 0.7152f + cb * 0.0722f;
-        float lum2 = lum * lum;
+      float lum = cr * 0.2126f + cg * 0.7152f + cb * 0.0722f;
+      float lum2 = lum * lum;
 #pragma unroll
-        for (int m = 1; m < LANES; m <<= 1) {
-          cr += __shfl_xor_sync(mask, cr, m, LANES);
-          cg += __shfl_xor_sync(mask, cg, m, LANES);
-          cb += __shfl_xor_sync(mask, cb, m, LANES);
-          lum += __shfl_xor_sync(mask, lum, m, LANES);
-          lum2 += __shfl_xor_sync(mask, lum2, m, LANES);
-        }
-        sr += cr; sg += cg; sb += cb; sum_l += lum; sum_l2 += lum2;
-        n = int(min(base + uint32_t(LANES), uint32_t(p.spp)));
-        if (p.adapt_min > 0 && n >= p.adapt_min && n > 1 && n % p.adapt_step == 0) {
-          float mean = sum_l / float(n);
-          float var = fmaxf(0.0f, (sum_l2 - sum_l * mean) / float(n - 1));
-          float thr = p.adapt_rel * mean + p.adapt_abs;
-          if (var < thr * thr) break;
-        }
+      for (int m = 1; m < LANES; m <<= 1) {
+        cr += __shfl_xor_sync(mask, cr, m, LANES);
+        cg += __shfl_xor_sync(mask, cg, m, LANES);
+        cb += __shfl_xor_sync(mask, cb, m, LANES);
+        lum += __shfl_xor_sync(mask, lum, m, LANES);
+        lum2 += __shfl_xor_sync(mask, lum2, m, LANES);
+      }
+      sr += cr; sg += cg; sb += cb; sum_l += lum; sum_l2 += lum2;
+      n = int(min(base + uint32_t(LANES), uint32_t(p.spp)));
+      if (p.adapt_min > 0 && n >= p.adapt_min && n > 1 && n % p.adapt_step == 0) {
+        float mean = sum_l / float(n);
+        float var = fmaxf(0.0f, (sum_l2 - sum_l * mean) / float(n - 1));
+        float thr = p.adapt_rel * mean + p.adapt_abs;
+        if (var < thr * thr) break;
       }
     }
     uint32_t st = pt.rng.state;
-    if (LANES > 1) {
-      const uint32_t group = (threadIdx.x & 31u) / LANES;
-      const uint32_t mask = LANES == 32 ? 0xffffffffu : (((1u << LANES) - 1u) << (group * LANES));
 #pragma unroll
-      for (int m = 1; m < LANES; m <<= 1) st ^= __shfl_xor_sync(mask, st, m, LANES);
-    }
+    for (int m = 1; m < LANES; m <<= 1) st ^= __shfl_xor_sync(mask, st, m, LANES);
     rays = pt.rays; nodes = pt.nodes; tests = pt.tests;
     if (lane == 0) {
       float cr = sr / float(n), cg = sg / float(n), cb = sb / float(n);
@@ -673,8 +647,7 @@ cudaError_t launch_render_paths(int lanes, const Scene& s, const Params& p, uint
   const uint64_t threads = uint64_t(p.width) * uint64_t(p.height) * uint64_t(lanes);
   const unsigned g = blocks_for(threads, 256);
   if (lanes == 32) k_render_paths<32><<<g, 256, 0, st>>>(s, p, seed, hdr, rgb, dbg, ctr, err);
-  else if (lanes == 8) k_render_paths<8><<<g, 256, 0, st>>>(s, p, seed, hdr, rgb, dbg, ctr, err);
-  else k_render_paths<1><<<g, 256, 0, st>>>(s, p, seed, hdr, rgb, dbg, ctr, err);
+  else k_render_paths<8><<<g, 256, 0, st>>>(s, p, seed, hdr, rgb, dbg, ctr, err);
   return cudaGetLastError();
 }
 

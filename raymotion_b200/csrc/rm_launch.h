@@ -12,8 +12,32 @@
 namespace rmd {
 
 // rm_kernels.cu
+// lanes 8 or 32
 cudaError_t launch_render_paths(int lanes, const Scene& s, const Params& p, uint64_t seed, float* hdr, uint8_t* rgb,
                                 uint32_t* dbg, unsigned long long* ctr, uint32_t* err, cudaStream_t st);
+
+// rm_paths.cu: the plain path tracer.  A chunk of the image (pixels [pixel0,
+// pixel0 + n_pixels)) runs segment by segment: rounds [round0, round1) of the
+// pixels still open.
+struct PathsArgs {
+  int pixel0, n_pixels, lanes, round0, round1;
+  float4* val;      // per round of the segment and lane slot: the sample's value
+  uint32_t* state;  // per lane slot: RNG state after the last finished segment
+  float4* gsum;     // per pixel: rgb and luminance sums of the earlier segments
+  float* gsl2;      // squared luminance
+  int* list[2];     // open pixels of even / odd segments (segment 0: all)
+  int* counts;      // per segment: open pixels
+  unsigned* next;   // per segment: tasks handed out
+  float* hdr;
+  uint8_t* rgb;
+  uint32_t* dbg;
+};
+long long paths_one_wave(int sms);  // lanes of one wave of resident blocks
+cudaError_t launch_paths(const Scene& s, const Params& p, uint64_t seed, const PathsArgs& a, int seg, int sms,
+                         unsigned long long* ctr, uint32_t* err, cudaStream_t st);
+// mode 0: every open pixel goes on, 1: those that fail the adaptive test, 2: none
+cudaError_t launch_paths_combine(const Params& p, const PathsArgs& a, int seg, int mode, int sms,
+                                 cudaStream_t st);
 // stage 0 generate, 1 spatial (temporal + spatial reuse), 2 shade
 cudaError_t launch_restir_stage(int stage, const Scene& s, const Params& p, uint64_t seed, const GBufSoA& gb,
                                 const ResSoA& ri, const ResSoA& rm, const GBufSoA& hg, const ResSoA& hr, float* hdr,
