@@ -102,11 +102,10 @@ cudaError_t launch_wavefront_shade3(const Scene& s, const Params& p, const GBufS
                                     unsigned long long* ctr, uint32_t* err, cudaStream_t st);
 // Run every path left in q (extension queue + queue c) to the end of its pixel.
 // wavefront_tail_capacity: the paths one wave of resident tail blocks holds.
-int wavefront_tail_capacity(bool opaque);
+int wavefront_tail_capacity(int sms);
 cudaError_t launch_wavefront_tail(const Scene& s, const Params& p, const GBufSoA& gb, const WfState& w,
                                   const WfQueues& q, int bound, float* hdr, uint32_t* dbg, unsigned long long* ctr,
-                                  unsigned long long* ctr_ext, unsigned long long* ctr_shd, uint32_t* err,
-                                  cudaStream_t st);
+                                  unsigned long long* ctr_tr, uint32_t* err, cudaStream_t st);
 
 // rm_batch.cu: many plain-path images (reference K1 / K2) rendered together
 // by one pool of path slots.  A pixel owns `lanes` consecutive lane slots (its

@@ -74,30 +74,11 @@ __global__ void __launch_bounds__(kPathThreads, kPathBlocks) k_paths(Scene s, Pa
   const int* list = seg == 0 ? nullptr : a.list[seg & 1];
   Tracer pt(s, p, err);
   PathRegs r;
-  bool active = false, more = true;
+  bool active = false, fresh = false, more = true;  // fresh: the next sample's camera ray is to be made
   uint32_t x = 0, y = 0, taken = 0;
   uint32_t slot = 0;   // pixel within the chunk x lanes + lane
   int si = 0, n = 0;   // sample; one lane: samples summed
   float sr = 0, sg = 0, sb = 0, sum_l = 0, sum_l2 = 0;
-  // the camera ray of the task's next sample (pathtrace.metal:754-756, :792-794; sample_sensor :729-737)
-  auto start = [&]() {
-    float sx, sy;
-    pt.jitter(x, y, sx, sy);
-    const rm_camera& cam = p.camera;
-    const float focal2 = cam.focal * cam.focal;
-    const float dist = 1.0f / sqrtf(sx * sx + (sy * sy + focal2));
-    const float tx = sx * dist, ty = sy * dist, tz = cam.focal * dist;
-    r.dx = tx * cam.m0 + (ty * cam.m1 + tz * cam.m2);
-    r.dy = tx * cam.m3 + (ty * cam.m4 + tz * cam.m5);
-    r.dz = tx * cam.m6 + (ty * cam.m7 + tz * cam.m8);
-    r.ox = cam.x; r.oy = cam.y; r.oz = cam.z;
-    r.ax = r.ay = r.az = 0.0f;
-    r.tx = r.ty = r.tz = 1.0f;
-    r.v = 0;
-    r.meta = kDelta;
-    r.last_pdf = 0.0f; r.psumW = 0.0f; r.pM = 0;
-    r.pbr = r.pbg = r.pbb = r.pbcos = 0.0f;
-  };
   for (;;) {
     const unsigned idle = __ballot_sync(full, !active);
     if (more && (__popc(idle) >= kRefill)) {
@@ -123,20 +104,40 @@ __global__ void __launch_bounds__(kPathThreads, kPathBlocks) k_paths(Scene s, Pa
         si = a.round0 * L + int(lane);
         n = 0;
         sr = sg = sb = sum_l = sum_l2 = 0.0f;
-        active = si < p.spp;
-        if (active) start();
-        else a.state[slot] = pt.rng.state;
+        active = fresh = si < p.spp;
+        if (!active) a.state[slot] = pt.rng.state;
       }
     }
     if (!__any_sync(full, active)) {
       if (!more) break;
       continue;
     }
+    if (fresh) {
+      // the camera ray of the next sample (pathtrace.metal:754-756, :792-794; sample_sensor :729-737)
+      float sx, sy;
+      pt.jitter(x, y, sx, sy);
+      const rm_camera& cam = p.camera;
+      const float focal2 = cam.focal * cam.focal;
+      const float dist = 1.0f / sqrtf(sx * sx + (sy * sy + focal2));
+      const float tx = sx * dist, ty = sy * dist, tz = cam.focal * dist;
+      r.dx = tx * cam.m0 + (ty * cam.m1 + tz * cam.m2);
+      r.dy = tx * cam.m3 + (ty * cam.m4 + tz * cam.m5);
+      r.dz = tx * cam.m6 + (ty * cam.m7 + tz * cam.m8);
+      r.ox = cam.x; r.oy = cam.y; r.oz = cam.z;
+      r.ax = r.ay = r.az = 0.0f;
+      r.tx = r.ty = r.tz = 1.0f;
+      r.v = 0;
+      r.meta = kDelta;
+      r.last_pdf = 0.0f; r.psumW = 0.0f; r.pM = 0;
+      r.pbr = r.pbg = r.pbb = r.pbcos = 0.0f;
+      fresh = false;
+    }
     if (active) {
       bool go = false;
       if (r.v < p.bounces) {
         // closest hit, through transparent crossings (pathtrace.metal:536-550)
-        const Hit hit = pt.cast_alpha_ray(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, kFar);
+        const Hit hit = NEE == 1 ? pt.cast_alpha_ray(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, kFar)
+                                 : pt.cast_ray(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, kFar);
         if (hit.tri >= 0) {
           bool has_shadow = false;
           float4 so, sd, c;
@@ -174,8 +175,7 @@ __global__ void __launch_bounds__(kPathThreads, kPathBlocks) k_paths(Scene s, Pa
           last = si >= p.spp || si / L >= a.round1;
           if (last) a.state[slot] = pt.rng.state;
         }
-        active = !last;
-        if (active) start();
+        active = fresh = !last;
       }
     }
   }

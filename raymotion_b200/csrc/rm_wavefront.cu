@@ -365,11 +365,11 @@ __global__ void __launch_bounds__(64, 20) k_wf_trace2(Scene s, WfState w, WfQueu
 }
 
 // One path of a shading queue: fold in its shadow ray, shade the vertex its
-// extension ray found (VK 0 opaque, 1 dielectric) or end it (VK 2), finish and
+// extension ray found (vk 0 opaque, 1 dielectric) or end it (vk 2), finish and
 // restart samples; ext / shd / fin tell which queues of the next wave take it.
 // NEE: the NEE variant of vertex() (2 in opaque scenes, 1 otherwise).
-template <int VK, int NEE>
-__device__ __forceinline__ void shade_path(const Scene& s, const Params& p, const GBufSoA& gb, const WfState& w, int id,
+template <int NEE>
+__device__ __forceinline__ void shade_path(int vk, const Scene& s, const Params& p, const GBufSoA& gb, const WfState& w, int id,
                                            float* __restrict__ hdr, uint32_t* __restrict__ dbg, uint32_t* err,
                                            bool& ext, bool& shd, bool& fin, uint32_t& samples) {
   const uint32_t x = uint32_t(id) % uint32_t(p.width), y = uint32_t(id) / uint32_t(p.width);
@@ -387,7 +387,7 @@ __device__ __forceinline__ void shade_path(const Scene& s, const Params& p, cons
     }
   }
   bool ended;
-  if (VK == 2) {
+  if (vk == 2) {
     ended = true;  // a miss ends the path; a finishing path has now folded in its last shadow ray
     r.meta &= ~(kExt | kFinish);
   } else {
@@ -397,7 +397,8 @@ __device__ __forceinline__ void shade_path(const Scene& s, const Params& p, cons
     const Hit hit = pt.attributes(tr, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz);
     bool has_shadow = false;
     float4 so, sd, c;
-    const bool go = vertex<VK, NEE>(pt, p, r, hit, has_shadow, so, sd, c);
+    const bool go = vk == 1 ? vertex<1, NEE>(pt, p, r, hit, has_shadow, so, sd, c)
+                            : vertex<0, NEE>(pt, p, r, hit, has_shadow, so, sd, c);
     if (has_shadow) {
       w.so[id] = so; w.sd[id] = sd; w.c[id] = c;
       r.meta |= kShadow;
@@ -436,7 +437,7 @@ __global__ void __launch_bounds__(256) k_wf_shade(Scene s, Params p, GBufSoA gb,
   uint32_t samples = 0;
   if (i < count) {
     id = queue[i];
-    shade_path<VK, NEE>(s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
+    shade_path<NEE>(VK, s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
   }
   append(nq.ext, nq.counts + kCntExt, ext, id);
   append(nq.shd, nq.counts + kCntShd, shd, id);
@@ -471,9 +472,9 @@ __global__ void __launch_bounds__(128, NEE == 2 ? 6 : 4) k_wf_shade3(Scene s, Pa
     if (bad_index(id, (long long)p.width * p.height, err, kSiteQueue)) id = -1;
   }
   if (id >= 0 && i < count) {
-    if (vk == 0) shade_path<0, NEE>(s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
-    else if (vk == 1) shade_path<1, NEE>(s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
-    else shade_path<2, NEE>(s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
+    if (vk == 0) shade_path<NEE>(0, s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
+    else if (vk == 1) shade_path<NEE>(1, s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
+    else shade_path<NEE>(2, s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
   }
   append(nq.ext, nq.counts + kCntExt, ext, id);
   append(nq.shd, nq.counts + kCntShd, shd, id);
@@ -481,69 +482,44 @@ __global__ void __launch_bounds__(128, NEE == 2 ? 6 : 4) k_wf_shade3(Scene s, Pa
   warp_add(ctr + 0, samples);
 }
 
-// One vertex step of a tail pixel, one thread per pixel: its extension ray,
-// its pending shadow ray and shade_path of the vertex type, in the waves'
-// order.  Returns true while the pixel has work left (ext: its next step
-// starts with an extension ray).  cnt: extension rays, nodes, tests; shadow
-// rays, nodes, tests.
-template <int NEE>
-__device__ __forceinline__ bool tail_step(const Scene& s, const Params& p, const GBufSoA& gb, const WfState& w, int id,
-                                          bool& ext, float* __restrict__ hdr, uint32_t* __restrict__ dbg,
-                                          uint32_t* err, uint32_t& samples, uint32_t* cnt) {
-  int vk = 2;
-  if (ext) {
-    const float4 o = w.o[id];
-    const float4 d = w.d[id];
-    const TraceResult r = traverse_quad<false>(s, o.x, o.y, o.z, d.x, d.y, d.z, kFar, err, cnt[1], cnt[2]);
-    ++cnt[0];
-    w.hit[id] = make_float4(r.t, r.u, r.v, __int_as_float(r.tri));
-    if (r.tri >= 0) vk = __ldg(&s.tris[r.tri].ior) > 1.0001f ? 1 : 0;
-  }
-  if (w.u[id].y & kShadow) {
-    const float4 o = w.so[id];
-    const float4 d = w.sd[id];
-    const TraceResult r = traverse_quad<true>(s, o.x, o.y, o.z, d.x, d.y, d.z, o.w, err, cnt[4], cnt[5]);
-    ++cnt[3];
-    w.occ[id] = r.tri >= 0 ? 1u : 0u;
-  }
-  bool shd = false, fin = false;
-  ext = false;
-  if (vk == 0) shade_path<0, NEE>(s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
-  else if (vk == 1) shade_path<1, NEE>(s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
-  else shade_path<2, NEE>(s, p, gb, w, id, hdr, dbg, err, ext, shd, fin, samples);
-  return ext || fin;
-}
-
-// The end of the wavefront loop, once few paths remain: each thread takes an
+// The end of the wavefront loop, once few paths remain: a thread takes an
 // unfinished pixel and runs it to the end with the waves' steps, in their
-// order (extension ray, pending shadow ray, shade_path of the vertex type), so
-// the pixel comes out the same, without a launch and a queue round trip per
-// vertex.  ctr: the stage counter of the tail's samples; ctr_ext / ctr_shd:
-// its traversals'.  Eight 64-thread blocks per SM (128 registers, ~200
-// bytes of spills): the tail is latency-bound and its path count is capped
-// to one wave of resident blocks, so more resident blocks can take the paths
-// over earlier (a capacity of 75.8 k instead of 56.8 k paths on 148 SMs; on
-// the 720p frame a tenth of the first wave, ~60.6 k, now sets the hand-off,
-// against 56.8 k before).  On the 720p frame:
-// six 64-thread blocks (168 registers) 330.5 against 327.3 M path samples/s
-// for three of 128 threads, and eight 334.1 against 331.2 M for six: a
-// point each, inside the run-to-run spread.
+// order (extension ray, shading, shadow ray), so the pixel comes out the same,
+// without a launch and a queue round trip per vertex.  Its state is read once
+// and stays in registers: a step that read and wrote it like a wave's took 68
+// ms (three parts summed) on the 720p frame against 61, the frame 114 against
+// 110 ms.  Bounded by the chain of the pixels with the most vertices left; four
+// 128-thread blocks per SM (128 registers, no spills to speak of): five 65 ms,
+// six 74.  ctr: the counters of the shading stage (samples); ctr_tr: the tail's
+// (rays, nodes and tests of both kinds).
+constexpr int kTailThreads = 128, kTailBlocks = 4;
+
 template <int NEE>
-__global__ void __launch_bounds__(64, 8) k_wf_tail(Scene s, Params p, GBufSoA gb, WfState w, WfQueues q,
+__global__ void __launch_bounds__(kTailThreads, kTailBlocks) k_wf_tail(Scene s, Params p, GBufSoA gb, WfState w, WfQueues q,
                                                  float* __restrict__ hdr, uint32_t* __restrict__ dbg,
-                                                 unsigned long long* ctr, unsigned long long* ctr_ext,
-                                                 unsigned long long* ctr_shd, uint32_t* err) {
+                                                 unsigned long long* ctr, unsigned long long* ctr_tr, uint32_t* err) {
   const int n_ext = q.counts[kCntExt], n_c = q.counts[kCntC];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  uint32_t samples = 0;
-  uint32_t cnt[6] = {0, 0, 0, 0, 0, 0};
+  Tracer pt(s, p, err);
+  PathRegs r;
+  uint32_t n = 0, samples = 0;
+  float sr = 0, sg = 0, sb = 0;
   bool active = i < n_ext + n_c;
   int id = 0;
-  bool ext = false;
   if (active) {
     id = i < n_ext ? q.ext[i] : q.qc[i - n_ext];
-    ext = i < n_ext;
     if (bad_index(id, (long long)p.width * p.height, err, kSiteTailQueue)) active = false;
+  }
+  if (active) {
+    load(w, uint32_t(id), r, pt.rng.state, n, sr, sg, sb);
+    if (r.meta & kShadow) {
+      const float4 o = w.so[id], d = w.sd[id];
+      if (!pt.shadow(o.x, o.y, o.z, d.x, d.y, d.z, o.w)) {
+        const float4 c = w.c[id];
+        r.ax += c.x; r.ay += c.y; r.az += c.z;
+      }
+    }
+    r.meta &= ~(kShadow | kFinish);
   }
   // each pass of the loop advances the pixel by one vertex, and a pixel has
   // at most spp x (depth + 2) vertices left: past that, flag and stop
@@ -553,16 +529,37 @@ __global__ void __launch_bounds__(64, 8) k_wf_tail(Scene s, Params p, GBufSoA gb
       atomicOr(err, kErrSteps);
       break;
     }
-    active = tail_step<NEE>(s, p, gb, w, id, ext, hdr, dbg, err, samples, cnt);
+    bool go = false;
+    if (r.meta & kExt) {
+      const Hit hit = pt.cast_ray(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, kFar);
+      if (hit.tri >= 0) {
+        bool has_shadow = false;
+        float4 so, sd, c;
+        go = hit.ior > 1.0001f ? vertex<1, NEE>(pt, p, r, hit, has_shadow, so, sd, c)
+                               : vertex<0, NEE>(pt, p, r, hit, has_shadow, so, sd, c);
+        if (has_shadow && !pt.shadow(so.x, so.y, so.z, sd.x, sd.y, sd.z, so.w)) {
+          r.ax += c.x; r.ay += c.y; r.az += c.z;
+        }
+      }
+    }
+    if (!go) {
+      const uint32_t n0 = n;
+      finish_sample(p, w, uint32_t(id), r, n, sr, sg, sb);
+      const uint32_t x = uint32_t(id) % uint32_t(p.width), y = uint32_t(id) / uint32_t(p.width);
+      if (start_samples(pt, p, gb, w, uint32_t(id), x, y, r, n, sr, sg, sb)) {
+        r.meta |= kExt;
+      } else {
+        write_pixel(p, uint32_t(id), (r.meta & kInd) != 0, n, sr, sg, sb, pt.rng.state, hdr, dbg);
+        active = false;
+      }
+      samples += n - n0;
+    }
   }
   __syncwarp();
   warp_add(ctr + 0, samples);
-  warp_add(ctr_ext + 1, cnt[0]);
-  warp_add(ctr_ext + 2, cnt[1]);
-  warp_add(ctr_ext + 3, cnt[2]);
-  warp_add(ctr_shd + 1, cnt[3]);
-  warp_add(ctr_shd + 2, cnt[4]);
-  warp_add(ctr_shd + 3, cnt[5]);
+  warp_add(ctr_tr + 1, pt.rays);
+  warp_add(ctr_tr + 2, pt.nodes);
+  warp_add(ctr_tr + 3, pt.tests);
 }
 
 }  // namespace
@@ -611,29 +608,15 @@ cudaError_t launch_wavefront_shade3(const Scene& s, const Params& p, const GBufS
   return cudaGetLastError();
 }
 
-int wavefront_tail_capacity(bool opaque) {
-  static int cap[2] = {0, 0};
-  int& c = cap[opaque ? 1 : 0];
-  if (c == 0) {
-    int dev = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, opaque ? k_wf_tail<2> : k_wf_tail<1>, 64, 0) !=
-            cudaSuccess)
-      return 0;
-    c = sms * per_sm * 64;
-  }
-  return c;
-}
+int wavefront_tail_capacity(int sms) { return sms * kTailBlocks * kTailThreads; }
 
 cudaError_t launch_wavefront_tail(const Scene& s, const Params& p, const GBufSoA& gb, const WfState& w,
                                   const WfQueues& q, int bound, float* hdr, uint32_t* dbg, unsigned long long* ctr,
-                                  unsigned long long* ctr_ext, unsigned long long* ctr_shd, uint32_t* err,
-                                  cudaStream_t st) {
+                                  unsigned long long* ctr_tr, uint32_t* err, cudaStream_t st) {
   if (bound <= 0) return cudaSuccess;
-  const unsigned g = unsigned((bound + 63) / 64);
-  if (p.opaque) k_wf_tail<2><<<g, 64, 0, st>>>(s, p, gb, w, q, hdr, dbg, ctr, ctr_ext, ctr_shd, err);
-  else k_wf_tail<1><<<g, 64, 0, st>>>(s, p, gb, w, q, hdr, dbg, ctr, ctr_ext, ctr_shd, err);
+  const unsigned g = unsigned((bound + kTailThreads - 1) / kTailThreads);
+  if (p.opaque) k_wf_tail<2><<<g, kTailThreads, 0, st>>>(s, p, gb, w, q, hdr, dbg, ctr, ctr_tr, err);
+  else k_wf_tail<1><<<g, kTailThreads, 0, st>>>(s, p, gb, w, q, hdr, dbg, ctr, ctr_tr, err);
   return cudaGetLastError();
 }
 

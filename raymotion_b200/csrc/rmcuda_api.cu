@@ -372,11 +372,20 @@ cudaError_t ensure_wavefront(rmcuda_ctx* c, size_t npix) {
 // the GPU mostly idle, above it the tail's one-thread-per-pixel loop is slower
 // than the waves), and no more than one wave of resident tail blocks holds (a
 // second wave of blocks would run after the first, doubling the tail).
+// Frames of few pixels are all tail: while the first wave's paths are few waves
+// of resident blocks, launching every step costs more than the waves' fuller
+// warps give (paths in one launch against waves: 333x187, 4 spp 1.78 / 2.37 ms;
+// 320x180, 64 spp 19.0 / 27.8; 480x270, 16 spp 8.1 / 10.0; 640x360, 16 spp 20.5
+// / 21.1; 1280x720, 64 spp 144 / 110): up to two resident waves.
 // RAYMOTION_CUDA_TAIL sets a fixed count; 0 keeps the waves to the end.
-static int tail_paths(int first_bound, bool opaque) {
+static int tail_paths(int first_bound, int sms) {
   const char* v = std::getenv("RAYMOTION_CUDA_TAIL");
   if (v) return std::max(0, std::atoi(v));
-  return std::min(first_bound / 10, rmd::wavefront_tail_capacity(opaque));
+  const int capacity = rmd::wavefront_tail_capacity(sms);
+  return first_bound <= 2 * capacity ? first_bound : std::min(first_bound / 10, capacity);
+}
+static bool all_tail(size_t npix, int sms) {
+  return !std::getenv("RAYMOTION_CUDA_TAIL") && npix <= 2 * size_t(rmd::wavefront_tail_capacity(sms));
 }
 
 cudaError_t run_wavefront_shade(rmcuda_ctx* c, const Scene& s, const Params& p, uint64_t seed, std::string& msg) {
@@ -401,7 +410,8 @@ cudaError_t run_wavefront_shade(rmcuda_ctx* c, const Scene& s, const Params& p, 
   // and 4 parts measured 310, 314 and 311 M path samples/s, one part 292 M).
   int parts = 3;
   if (const char* v = std::getenv("RAYMOTION_CUDA_STREAMS")) parts = std::max(1, std::min(kWfParts, std::atoi(v)));
-  if (!merged || p.height < parts) parts = 1;
+  const bool direct = all_tail(npix, c->sms);  // known without reading the first wave's queues
+  if (!merged || p.height < parts || direct) parts = 1;
   if (parts > 1 && !c->ev_fork && cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
     parts = 1;
@@ -479,7 +489,15 @@ cudaError_t run_wavefront_shade(rmcuda_ctx* c, const Scene& s, const Params& p, 
   int bound[kWfParts] = {};
   std::chrono::steady_clock::time_point t0;
   int tail = 0;
-  for (uint64_t wave = 0;; wave += kBatch) {
+  if (direct) {
+    t0 = std::chrono::steady_clock::now();
+    e = staged2(c, RM_STAGE_WF_TAIL, [&] {
+      return launch_wavefront_tail(s, p, c->gb.view(), w, q[0][0], int(npix), c->hdr.as<float>(), c->dbg.as<uint32_t>(),
+                                   ctr + 4 * RM_STAGE_WF_SHADE, ctr + 4 * RM_STAGE_WF_TAIL, err, c->stream);
+    });
+    if (e != cudaSuccess) { msg = cuda_msg("wavefront tail failed", e); return e; }
+  }
+  for (uint64_t wave = 0; !direct; wave += kBatch) {
     if (wave > max_waves) { msg = "wavefront did not drain"; return cudaErrorLaunchFailure; }
     for (int h = 0; h < parts; ++h)
       if (!done[h] &&
@@ -507,7 +525,7 @@ cudaError_t run_wavefront_shade(rmcuda_ctx* c, const Scene& s, const Params& p, 
     const auto now = std::chrono::steady_clock::now();
     if (wave == 0) {
       t0 = now;
-      tail = tail_paths(b_all, p.opaque != 0) / parts;
+      tail = tail_paths(b_all, c->sms) / parts;
     }
     c->wave_log.insert(c->wave_log.end(), {b_all, ext_all, shd_all,
                                            int(std::chrono::duration_cast<std::chrono::microseconds>(now - t0).count())});
@@ -521,7 +539,7 @@ cudaError_t run_wavefront_shade(rmcuda_ctx* c, const Scene& s, const Params& p, 
           // the tail's traversals are counted with the tail (both kinds in its slot)
           return launch_wavefront_tail(s, p, c->gb.view(), w, q[h][cur[h]], bound[h], c->hdr.as<float>(),
                                        c->dbg.as<uint32_t>(), ctr + 4 * RM_STAGE_WF_SHADE, ctr + 4 * RM_STAGE_WF_TAIL,
-                                       ctr + 4 * RM_STAGE_WF_TAIL, err, sts[h]);
+                                       err, sts[h]);
         });
         if (e != cudaSuccess) { msg = cuda_msg("wavefront tail failed", e); return e; }
         done[h] = true;
