@@ -184,13 +184,15 @@ void batch_occupancy(int& aux, int& trace, int& shade);
 // rm_adjoint.cu: path-replay adjoint of the plain frame (adds g . dC/dparams
 // into grad, n_mat x 8 floats: albedo rgb, rough, emission rgb, ior).
 cudaError_t launch_adjoint(int lanes, const Scene& s, const Params& p, uint64_t seed, const int32_t* tri_mat,
-                           int n_mat, const float* dLdI, float* grad, unsigned long long* ctr, uint32_t* err,
-                           cudaStream_t st);
+                           int n_mat, const float* dLdI, float* grad, unsigned* next, int sms, unsigned long long* ctr,
+                           uint32_t* err, cudaStream_t st);
+// `next` (device): the hand-out counter.
 // The adjoint of the ReSTIR shade from the frame's G-buffer and merged
-// reservoirs (one thread per pixel).
+// reservoirs.
 cudaError_t launch_adjoint_restir(const Scene& s, const Params& p, uint64_t seed, const GBufSoA& gb, const ResSoA& rm,
                                   const int32_t* tri_mat, int n_mat, const float* dLdI, const float* dLdalb,
-                                  float* grad, unsigned long long* ctr, uint32_t* err, cudaStream_t st);
+                                  float* grad, unsigned* next, int sms, unsigned long long* ctr, uint32_t* err,
+                                  cudaStream_t st);
 // rm_denoise_adjoint.cu: dL/d(ReSTIR shade HDR) and dL/d(G-buffer albedo) from
 // dL/d(denoised image), the G-buffer geometry and history colour of the frame
 // held; scratch holds 14 floats per pixel.

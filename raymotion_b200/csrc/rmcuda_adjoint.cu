@@ -83,6 +83,8 @@ int rmcuda_backward(rmcuda_ctx* c, const rmcuda_scene* scene, const rm_camera* c
   cudaSetDevice(c->device);
   const DevScene& sc = scene->d;
   if (sc.n_materials <= 0) { set_err(err, errcap, "scene has no materials (rmcuda_scene_set_materials)"); return RM_ERR_INVALID; }
+  // pixel lanes that the kernel has handed out
+  unsigned* next = reinterpret_cast<unsigned*>(c->ctr.as<unsigned long long>() + 4 * RM_STAGE_COUNT);
   Plan pl = make_plan(sc, *cam, *cfg);
   if (pl.use_spatial) {
     // the ReSTIR chain: K5 replayed from the checkpoint the frame left in the
@@ -129,7 +131,7 @@ int rmcuda_backward(rmcuda_ctx* c, const rmcuda_scene* scene, const rm_camera* c
     pl.p.hasHistory = 0;
     e = staged(c, RM_STAGE_ADJOINT, [&] {
       return launch_adjoint_restir(scene_view(sc), pl.p, seed, c->hg.view(), c->hres.view(), sc.tri_mat.as<int32_t>(),
-                                   sc.n_materials, dl_hdr, dl_alb, d_grad,
+                                   sc.n_materials, dl_hdr, dl_alb, d_grad, next, c->sms,
                                    c->ctr.as<unsigned long long>() + 4 * RM_STAGE_ADJOINT, c->err.as<uint32_t>(),
                                    c->stream);
     });
@@ -142,8 +144,8 @@ int rmcuda_backward(rmcuda_ctx* c, const rmcuda_scene* scene, const rm_camera* c
   }
   cudaError_t e = staged(c, RM_STAGE_ADJOINT, [&] {
     return launch_adjoint(pl.lanes, scene_view(sc), pl.p, seed, sc.tri_mat.as<int32_t>(), sc.n_materials,
-                          d_dL_dimage, d_grad, c->ctr.as<unsigned long long>() + 4 * RM_STAGE_ADJOINT,
-                          c->err.as<uint32_t>(), c->stream);
+                          d_dL_dimage, d_grad, next, c->sms,
+                          c->ctr.as<unsigned long long>() + 4 * RM_STAGE_ADJOINT, c->err.as<uint32_t>(), c->stream);
   });
   if (e != cudaSuccess) { set_err(err, errcap, cuda_msg("adjoint launch failed", e)); return RM_ERR_CUDA; }
   return RM_OK;

@@ -855,7 +855,7 @@ int rmcuda_create(rmcuda_ctx** out, int device, char* err, size_t errcap) {
   cudaError_t e = cudaSetDevice(device);
   pool_open(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = c->ctr.reserve(RM_STAGE_COUNT * 32);
+  if (e == cudaSuccess) e = c->ctr.reserve(RM_STAGE_COUNT * 32 + 32);  // the adjoint's hand-out counter behind the stages'
   if (e == cudaSuccess) e = c->err.reserve(4);
   if (e == cudaSuccess) e = cudaMemset(c->ctr.ptr, 0, RM_STAGE_COUNT * 32);
   if (e == cudaSuccess) e = cudaMemset(c->err.ptr, 0, 4);
