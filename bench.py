@@ -275,7 +275,7 @@ def batch_compare(args, backend, torch, stream, dev, world):
     log-uniform over [1k, 2M], resolutions from {256x256, 640x360, 1280x720,
     1920x1080}, spp from {4, 16, 64}, depth 8-12, plain path.  Serial: the
     single-frame policy per scene object (rmcuda_render_scene_async), all
-    enqueued back to back; batched: rmcuda_render_batch with the settings
+    enqueued back to back; batched: rmcuda_render_batch with the pool settings
     rmcuda_batch_tune picked (tuning is untimed).  Both produce the same
     images bit for bit (checked), so their relMSE is equal."""
     from raymotion_b200 import BatchItem

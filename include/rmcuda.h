@@ -317,7 +317,9 @@ typedef struct rm_batch_tuning {
 } rm_batch_tuning;
 
 /* Render many images of (possibly different) scenes, views, resolutions,
- * sample counts and depths together in one pool of path slots.  Each image is
+ * sample counts and depths: on several streams, or together in one pool of
+ * path slots (more than 32 images of fewer than 65,536 samples, those).  The
+ * tuning applies to the pool.  Each image is
  * what the plain single-frame chain gives it: render_paths (K1) or the 8/32
  * lane kernel (K2) of pathtrace.metal:739-815 with the lane rule of
  * metal.mm:390-394, adaptive sampling and clamp, bit for bit equal to
@@ -331,8 +333,8 @@ int rmcuda_render_batch(rmcuda_ctx* ctx, const rm_batch_item* items, int32_t n, 
  * in `out` (may be NULL).  Leaves partial images in the items' buffers. */
 int rmcuda_batch_tune(rmcuda_ctx* ctx, const rm_batch_item* items, int32_t n, rm_batch_tuning* out,
                       char* err, size_t errcap);
-/* Progress of the last batch: for each check between graph replays (every
- * graph_waves waves, or 8 without a graph) the live lane slots (queued to
+/* Progress of the last batch's pool: for each check between graph replays
+ * (every graph_waves waves, or 8 without a graph) the live lane slots (queued to
  * start, trace or finish) and the extension rays queued, at most `cap`
  * records (2 ints each) written.  Returns the number of records. */
 int rmcuda_batch_log(rmcuda_ctx* ctx, int32_t* out, int32_t cap);

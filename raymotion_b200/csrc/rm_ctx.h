@@ -104,6 +104,7 @@ struct BatchPool {
   cudaGraphExec_t exec = nullptr;
   uint64_t waves = 0;
   std::vector<int> wave_log;  // last batch: (live slots, extension rays) per check
+  DevBuf paths[rmd::kStreams - 1];  // workspaces of the images rendered on the side streams
   void release();
 };
 
@@ -171,8 +172,8 @@ struct rmcuda_ctx {
   rmd::DevBuf wq[10 * rmd::kWfParts + 1];
   int* h_counts = nullptr;  // pinned: two reads of the parts' queue lengths (2 x kWfParts x kCntSlots)
   cudaEvent_t ev_counts[2][rmd::kWfParts] = {};  // the end of each of those reads
-  cudaStream_t side_stream[rmd::kWfParts - 1] = {};
-  cudaEvent_t ev_fork = nullptr, ev_join[rmd::kWfParts - 1] = {};
+  cudaStream_t side_stream[rmd::kStreams - 1] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[rmd::kStreams - 1] = {};
   size_t wf_cap = 0;
   uint64_t waves = 0;
   std::vector<int> wave_log;  // last frame: (act, ext, shd, us) per count read
@@ -263,5 +264,31 @@ Plan make_plan(const DevScene& sc, const rm_camera& cam, const rm_config& cfg);
 int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_config& cfg, uint64_t seed,
                   uint8_t* d_rgb, std::string& msg);
 int check_device_error(rmcuda_ctx* c, std::string& msg);
+
+// How run_paths takes one image: its segments, and the layout of its workspace.
+struct PathsPlan {
+  std::vector<int> ends;   // the segments' last rounds + 1
+  std::vector<bool> test;  // the adaptive test follows
+  bool one_launch = false; // the lane kernel, without a workspace
+  long long chunk = 0;     // pixels at a time
+  size_t val = 0, state = 0, gsum = 0, gsl2 = 0, list[2] = {0, 0}, counts = 0, bytes = 0;
+};
+struct PathsTarget {
+  rmd::DevBuf& ws;
+  cudaStream_t stream;
+  float* hdr;
+  uint8_t* rgb;
+  uint32_t* dbg;
+  int stage;   // whose counters the image's work adds to
+  bool timed;  // by the profiler, on the context stream
+};
+// `samples`: the most whose values the workspace holds.
+PathsPlan plan_paths(rmcuda_ctx* c, const rmd::Params& p, int lanes, long long samples);
+// The plain chain of one image (rm_paths.cu), enqueued on t.stream.
+cudaError_t run_paths(rmcuda_ctx* c, const rmd::Scene& s, const rmd::Params& p, int lanes, uint64_t seed,
+                      const PathsPlan& q, const PathsTarget& t);
+// Create the context's streams beside its own, up to `parts` in all; lowers
+// `parts` to what there is.
+void side_streams(rmcuda_ctx* c, int& parts);
 
 }  // namespace rmapi

@@ -78,6 +78,9 @@ struct WfQueues {
 // The frame's pixels in up to kWfParts parts by row (row y in part y mod
 // parts), each with its own queues.
 constexpr int kWfParts = 4;
+// Streams of a context, its own among them, for a batch's images (4: 12.6 ms
+// for eight images of 45 k to 14.7 M samples, 8: 12.0).
+constexpr int kStreams = 8;
 struct WfParts {
   WfQueues q[kWfParts];
   int parts;

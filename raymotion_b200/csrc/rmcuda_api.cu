@@ -412,18 +412,7 @@ cudaError_t run_wavefront_shade(rmcuda_ctx* c, const Scene& s, const Params& p, 
   if (const char* v = std::getenv("RAYMOTION_CUDA_STREAMS")) parts = std::max(1, std::min(kWfParts, std::atoi(v)));
   const bool direct = all_tail(npix, c->sms);  // known without reading the first wave's queues
   if (!merged || p.height < parts || direct) parts = 1;
-  if (parts > 1 && !c->ev_fork && cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess) {
-    cudaGetLastError();
-    parts = 1;
-  }
-  for (int h = 1; h < parts; ++h)
-    if (!c->side_stream[h - 1] &&
-        (cudaStreamCreateWithFlags(&c->side_stream[h - 1], cudaStreamNonBlocking) != cudaSuccess ||
-         cudaEventCreateWithFlags(&c->ev_join[h - 1], cudaEventDisableTiming) != cudaSuccess)) {
-      cudaGetLastError();
-      parts = h;
-      break;
-    }
+  side_streams(c, parts);
   cudaStream_t sts[kWfParts];
   for (int h = 0; h < kWfParts; ++h) sts[h] = h == 0 || h >= parts ? c->stream : c->side_stream[h - 1];
   // on an early return (an error), the other parts' queued work finishes
@@ -626,84 +615,111 @@ cudaError_t ensure_frame(rmcuda_ctx* c, size_t npix, bool restir) {
 constexpr long long kPathChunk = 16ll << 20;
 constexpr int kPathSamples = 4096;  // most samples of a pixel in one segment
 
-cudaError_t run_paths(rmcuda_ctx* c, const Scene& s, const Params& p, int lanes, uint64_t seed, uint8_t* d_rgb) {
+PathsPlan plan_paths(rmcuda_ctx* c, const Params& p, int lanes, long long samples) {
+  PathsPlan q;
   const long long npix = (long long)p.width * p.height;
   const int rounds = (p.spp + lanes - 1) / lanes;
-  std::vector<int> ends;  // the segments' last rounds + 1
-  std::vector<bool> test;
   for (int r = 0; lanes > 1 && r + 1 < rounds; ++r) {
     const int n = (r + 1) * lanes;
     const bool t = p.adapt_min > 0 && n >= p.adapt_min && n % p.adapt_step == 0;
-    if (t || r + 1 - (ends.empty() ? 0 : ends.back()) >= kPathSamples / lanes) {
-      ends.push_back(r + 1);
-      test.push_back(t);
+    if (t || r + 1 - (q.ends.empty() ? 0 : q.ends.back()) >= kPathSamples / lanes) {
+      q.ends.push_back(r + 1);
+      q.test.push_back(t);
     }
   }
-  ends.push_back(lanes > 1 ? rounds : 1);
-  test.push_back(false);
+  q.ends.push_back(lanes > 1 ? rounds : 1);
+  q.test.push_back(false);
   int longest = 1;
-  for (size_t k = 0; k < ends.size(); ++k) longest = std::max(longest, ends[k] - (k ? ends[k - 1] : 0));
-  const size_t segs = ends.size();
+  for (size_t k = 0; k < q.ends.size(); ++k) longest = std::max(longest, q.ends[k] - (k ? q.ends[k - 1] : 0));
+  const size_t segs = q.ends.size();
   // When every lane has a thread of its own and the adaptive test cuts the
   // frame into segments, the one-launch lane kernel stays: its warps pass the
   // test without waiting for the slowest path of the frame (64x36, 256 spp, 2 k
   // triangles 1.04 ms against 2.05; 128x72 3.10 against 3.13; 160x100 4.43
   // against 4.02).
-  if (segs > 1 && npix * lanes <= paths_one_wave(c->sms))
-    return staged(c, RM_STAGE_PLAIN, [&] {
-      return launch_render_paths(lanes, s, p, seed, c->hdr.as<float>(), d_rgb, c->dbg.as<uint32_t>(),
-                                 c->ctr.as<unsigned long long>() + 4 * RM_STAGE_PLAIN, c->err.as<uint32_t>(), c->stream);
-    });
+  q.one_launch = segs > 1 && npix * lanes <= paths_one_wave(c->sms);
+  if (q.one_launch) return q;
   const long long per_pixel = (long long)lanes * longest;
-  const long long chunk = lanes == 1 ? npix : std::min(npix, std::max<long long>(1, kPathChunk / per_pixel));
+  q.chunk = lanes == 1 ? npix : std::min(npix, std::max<long long>(1, samples / per_pixel));
   // one allocation: values, states, sums, lists, counters
-  size_t off = 0;
   auto take = [&](size_t bytes) {
-    const size_t at = off;
-    off += (bytes + 255) & ~size_t(255);
+    const size_t at = q.bytes;
+    q.bytes += (bytes + 255) & ~size_t(255);
     return at;
   };
-  const size_t px = size_t(chunk), several = lanes > 1 ? 1 : 0, multi = segs > 1 ? several : 0;
-  const size_t o_val = take(several * px * size_t(per_pixel) * sizeof(float4));
-  const size_t o_state = take(px * size_t(lanes) * sizeof(uint32_t));
-  const size_t o_gsum = take(multi * px * sizeof(float4)), o_gsl2 = take(multi * px * sizeof(float));
-  const size_t o_list0 = take(multi * px * sizeof(int)), o_list1 = take(multi * px * sizeof(int));
-  const size_t o_cnt = take((segs + 1) * 2 * sizeof(int));
-  cudaError_t e = c->paths.reserve(off);
+  const size_t px = size_t(q.chunk), several = lanes > 1 ? 1 : 0, multi = segs > 1 ? several : 0;
+  q.val = take(several * px * size_t(per_pixel) * sizeof(float4));
+  q.state = take(px * size_t(lanes) * sizeof(uint32_t));
+  q.gsum = take(multi * px * sizeof(float4));
+  q.gsl2 = take(multi * px * sizeof(float));
+  q.list[0] = take(multi * px * sizeof(int));
+  q.list[1] = take(multi * px * sizeof(int));
+  q.counts = take((segs + 1) * 2 * sizeof(int));
+  return q;
+}
+
+cudaError_t run_paths(rmcuda_ctx* c, const Scene& s, const Params& p, int lanes, uint64_t seed,
+                      const PathsPlan& q, const PathsTarget& t) {
+  const long long npix = (long long)p.width * p.height;
+  unsigned long long* ctr = c->ctr.as<unsigned long long>() + 4 * t.stage;
+  uint32_t* err = c->err.as<uint32_t>();
+  auto launch = [&](auto&& fn) {
+    if (t.timed) return staged(c, t.stage, fn);
+    c->launches += 1;
+    return fn();
+  };
+  if (q.one_launch)
+    return launch([&] { return launch_render_paths(lanes, s, p, seed, t.hdr, t.rgb, t.dbg, ctr, err, t.stream); });
+  cudaError_t e = t.ws.reserve(q.bytes);
   if (e != cudaSuccess) return e;
-  char* base = c->paths.as<char>();
+  const size_t segs = q.ends.size();
+  char* base = t.ws.as<char>();
   PathsArgs a{};
   a.lanes = lanes;
-  a.val = reinterpret_cast<float4*>(base + o_val);
-  a.state = reinterpret_cast<uint32_t*>(base + o_state);
-  a.gsum = reinterpret_cast<float4*>(base + o_gsum);
-  a.gsl2 = reinterpret_cast<float*>(base + o_gsl2);
-  a.list[0] = reinterpret_cast<int*>(base + o_list0);
-  a.list[1] = reinterpret_cast<int*>(base + o_list1);
-  a.counts = reinterpret_cast<int*>(base + o_cnt);
+  a.val = reinterpret_cast<float4*>(base + q.val);
+  a.state = reinterpret_cast<uint32_t*>(base + q.state);
+  a.gsum = reinterpret_cast<float4*>(base + q.gsum);
+  a.gsl2 = reinterpret_cast<float*>(base + q.gsl2);
+  a.list[0] = reinterpret_cast<int*>(base + q.list[0]);
+  a.list[1] = reinterpret_cast<int*>(base + q.list[1]);
+  a.counts = reinterpret_cast<int*>(base + q.counts);
   a.next = reinterpret_cast<unsigned*>(a.counts + segs + 1);
-  a.hdr = c->hdr.as<float>();
-  a.rgb = d_rgb;
-  a.dbg = c->dbg.as<uint32_t>();
-  for (long long p0 = 0; p0 < npix; p0 += chunk) {
+  a.hdr = t.hdr;
+  a.rgb = t.rgb;
+  a.dbg = t.dbg;
+  for (long long p0 = 0; p0 < npix; p0 += q.chunk) {
     a.pixel0 = int(p0);
-    a.n_pixels = int(std::min(chunk, npix - p0));
-    if ((e = cudaMemsetAsync(a.counts, 0, (segs + 1) * 2 * sizeof(int), c->stream)) != cudaSuccess) return e;
+    a.n_pixels = int(std::min(q.chunk, npix - p0));
+    if ((e = cudaMemsetAsync(a.counts, 0, (segs + 1) * 2 * sizeof(int), t.stream)) != cudaSuccess) return e;
     for (size_t k = 0; k < segs; ++k) {
-      a.round0 = k ? ends[k - 1] : 0;
-      a.round1 = ends[k];
-      e = staged(c, RM_STAGE_PLAIN, [&] {
-        cudaError_t q = launch_paths(s, p, seed, a, int(k), c->sms, c->ctr.as<unsigned long long>() + 4 * RM_STAGE_PLAIN,
-                                     c->err.as<uint32_t>(), c->stream);
-        if (q == cudaSuccess && lanes > 1) c->launches += 1;
-        if (q == cudaSuccess && lanes > 1)
-          q = launch_paths_combine(p, a, int(k), k + 1 == segs ? 2 : test[k] ? 1 : 0, c->sms, c->stream);
-        return q;
+      a.round0 = k ? q.ends[k - 1] : 0;
+      a.round1 = q.ends[k];
+      e = launch([&] {
+        cudaError_t r = launch_paths(s, p, seed, a, int(k), c->sms, ctr, err, t.stream);
+        if (r == cudaSuccess && lanes > 1) c->launches += 1;
+        if (r == cudaSuccess && lanes > 1)
+          r = launch_paths_combine(p, a, int(k), k + 1 == segs ? 2 : q.test[k] ? 1 : 0, c->sms, t.stream);
+        return r;
       });
       if (e != cudaSuccess) return e;
     }
   }
   return cudaSuccess;
+}
+
+void side_streams(rmcuda_ctx* c, int& parts) {
+  if (parts > 1 && !c->ev_fork && cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    parts = 1;
+  }
+  for (int h = 1; h < parts; ++h)
+    if (!c->side_stream[h - 1] &&
+        (cudaStreamCreateWithFlags(&c->side_stream[h - 1], cudaStreamNonBlocking) != cudaSuccess ||
+         cudaEventCreateWithFlags(&c->ev_join[h - 1], cudaEventDisableTiming) != cudaSuccess)) {
+      cudaGetLastError();
+      parts = h;
+      break;
+    }
 }
 
 // Enqueue one frame of the resident scene.  d_rgb (device) receives the
@@ -731,7 +747,8 @@ int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_co
   uint32_t* err = c->err.as<uint32_t>();
   if (!pl.use_spatial) {
     c->last_chain = pl.lanes;
-    e = run_paths(c, s, p, pl.lanes, seed, d_rgb);
+    e = run_paths(c, s, p, pl.lanes, seed, plan_paths(c, p, pl.lanes, kPathChunk),
+                  PathsTarget{c->paths, st, c->hdr.as<float>(), d_rgb, c->dbg.as<uint32_t>(), RM_STAGE_PLAIN, true});
     if (e != cudaSuccess) { msg = cuda_msg("render_paths launch failed", e); return RM_ERR_CUDA; }
     c->last_final = c->hdr.as<float>();
   } else {
@@ -884,7 +901,7 @@ void rmcuda_destroy(rmcuda_ctx* c) {
                     &c->adj_scratch, &c->differ, &c->ctr_save, &c->paths})
     b->release();
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
-  for (int h = 0; h < kWfParts - 1; ++h) {
+  for (int h = 0; h < kStreams - 1; ++h) {
     if (c->side_stream[h]) cudaStreamDestroy(c->side_stream[h]);
     if (c->ev_join[h]) cudaEventDestroy(c->ev_join[h]);
   }

@@ -1,9 +1,10 @@
 // rmcuda_batch.cu - the C ABI of scene objects and batched rendering
 // (include/rmcuda.h): many images, each the reference's plain single-frame
 // chain (pathtrace.metal:739-815 with the policy of metal.mm:146-170,
-// :390-394), rendered together by the persistent wavefront of rm_batch.cu.
+// :390-394), rendered by the plain frame's kernels on several streams or, where
+// many are small, together by the persistent wavefront of rm_batch.cu.
 //
-// Host side of a batch: build the job table (one entry per image, largest
+// Host side of the latter: build the job table (one entry per image, largest
 // first so the pool drains on small images), reset the pool, then launch
 // waves, captured once into a CUDA graph of `graph_waves` waves and replayed
 // until the queue lengths read back after a replay show no work left.  The
@@ -31,6 +32,7 @@ void rmapi::BatchPool::release() {
   jobs.release();
   tile_begin.release();
   next_tile.release();
+  for (DevBuf& b : paths) b.release();
   if (exec) cudaGraphExecDestroy(exec);
   exec = nullptr;
   if (h_counts) cudaFreeHost(h_counts);
@@ -106,19 +108,40 @@ void tile_shape(int lanes, int shape, int& tw, int& th) {
   }
 }
 
+// Images go through the plain frame's kernels (rm_paths.cu), on kStreams
+// streams: paths stay in registers there, where a wave of the pool stores and
+// reloads each path's state and ends with its slowest warps (eight images of
+// 45 k to 14.7 M samples 24.4 -> 12.0 ms; one of 64x36, 4 spp 1.4 -> 0.2; 64 of
+// 160x90, 16 spp 14.5 -> 10.3).  An image costs about 70 us of launches then,
+// which the pool pays once (2.2 to 2.5 ms a batch, then about 1.1 ns a sample),
+// so many small ones stay with the pool: more than kFewSmall images of fewer
+// than kOwnSamples samples (256 of 64x36, 4 spp 17.4 ms alone, 6.5 in the pool;
+// of 64x36, 16 spp 14.2 and 11.0; of 160x90, 4 spp 21.7 and 19.0; 64 of each 4.3
+// / 3.9, 3.6 / 4.4 and 5.4 / 6.7).
+constexpr double kOwnSamples = 65536.0;
+constexpr int kFewSmall = 32;
+constexpr long long kOwnChunk = 4ll << 20;  // samples whose values a stream holds (16 M: 11.9 ms)
+
+bool small_image(const rm_config& cfg) {
+  return double(cfg.width) * double(cfg.height) * double(cfg.spp) < kOwnSamples;
+}
+
 struct Prepared {
-  std::vector<BtJob> jobs;  // largest first
+  std::vector<BtJob> own;   // images rendered alone (run_own), largest first
+  std::vector<BtJob> jobs;  // the pool's, largest first
   std::vector<int> tile_begin;
   int total_tiles = 0;
   uint64_t max_waves = 0;
 };
 
-int prepare(rmcuda_ctx* c, const rm_batch_item* items, int n, int shape, int width, Prepared& out,
+int prepare(rmcuda_ctx* c, const rm_batch_item* items, int n, int shape, int width, bool pool_only, Prepared& out,
             std::string& msg) {
   if (n < 0 || (n > 0 && !items)) { msg = "invalid batch"; return RM_ERR_INVALID; }
   std::vector<std::pair<double, int>> order;
   std::vector<BtJob> jobs(static_cast<size_t>(n));
-  int max_rounds = 1, max_bounces = 0;
+  std::vector<char> alone(static_cast<size_t>(n));
+  int max_rounds = 1, max_bounces = 0, n_small = 0;
+  for (int i = 0; i < n; ++i) n_small += small_image(items[i].config) ? 1 : 0;
   for (int i = 0; i < n; ++i) {
     const rm_batch_item& it = items[i];
     const rm_config& cfg = it.config;
@@ -142,7 +165,8 @@ int prepare(rmcuda_ctx* c, const rm_batch_item* items, int n, int shape, int wid
     std::memset(&J, 0, sizeof(J));
     // the collapse is a cache of the scene object, built once under the context lock
     rmd::DevBvh& bvh = const_cast<rmcuda_scene*>(it.scene)->d.bvh;
-    if (width == 8 && bvh.n_wide == 0 && bvh.n_records > 0) {
+    const bool own = !pool_only && (n_small <= kFewSmall || !small_image(cfg));
+    if (!own && width == 8 && bvh.n_wide == 0 && bvh.n_records > 0) {
       // collapse this scene's binary BVH on first use (none if too deep: the
       // job then traverses the binary BVH, which gives the same hits)
       const cudaError_t e = rmd::build_wide(bvh, c->stream);
@@ -162,23 +186,31 @@ int prepare(rmcuda_ctx* c, const rm_batch_item* items, int n, int shape, int wid
     tile_shape(pl.lanes, shape, J.tile_w, J.tile_h);
     J.tiles_x = (cfg.width + J.tile_w - 1) / J.tile_w;
     J.tiles = J.tiles_x * ((cfg.height + J.tile_h - 1) / J.tile_h);
+    const double cost = double(cfg.width) * double(cfg.height) * double(cfg.spp) * double(cfg.max_bounces + 1);
+    order.push_back({-cost, i});
+    alone[size_t(i)] = own;
+    if (own) continue;
     const int rounds = (cfg.spp + pl.lanes - 1) / pl.lanes;
     max_rounds = std::max(max_rounds, rounds);
     max_bounces = std::max(max_bounces, cfg.max_bounces);
-    const double cost = double(cfg.width) * double(cfg.height) * double(cfg.spp) * double(cfg.max_bounces + 1);
-    order.push_back({-cost, i});
   }
   std::stable_sort(order.begin(), order.end());
+  out.own.clear();
   out.jobs.clear();
   out.tile_begin.clear();
-  int64_t t = 0;
+  int64_t t = 0, all = 0;
   for (auto& o : order) {
     BtJob J = jobs[size_t(o.second)];
+    all += J.tiles;
+    if (all > (int64_t(1) << 30)) { msg = "batch too large"; return RM_ERR_INVALID; }
+    if (alone[size_t(o.second)]) {
+      out.own.push_back(J);
+      continue;
+    }
     J.tile_begin = int(t);
     out.jobs.push_back(J);
     out.tile_begin.push_back(int(t));
     t += J.tiles;
-    if (t > (int64_t(1) << 30)) { msg = "batch too large"; return RM_ERR_INVALID; }
   }
   out.total_tiles = int(t);
   // A chunk finishes its tile within rounds x (bounces + 2) waves and is
@@ -340,6 +372,61 @@ int run_batch(rmcuda_ctx* c, const Prepared& P, const rm_batch_tuning& tune, Win
   return rc;
 }
 
+// The images rendered alone, each on the stream that has the least work so far
+// (one image's last paths leave room for another's).
+int run_own(rmcuda_ctx* c, const std::vector<BtJob>& jobs, std::string& msg) {
+  if (jobs.empty()) return RM_OK;
+  int parts = int(std::min<size_t>(jobs.size(), kStreams));
+  side_streams(c, parts);
+  cudaStream_t sts[kStreams];
+  DevBuf* ws[kStreams];
+  for (int h = 0; h < parts; ++h) {
+    sts[h] = h == 0 ? c->stream : c->side_stream[h - 1];
+    ws[h] = h == 0 ? &c->paths : &c->batch.paths[h - 1];
+  }
+  std::vector<PathsPlan> plans;
+  for (const BtJob& J : jobs) plans.push_back(plan_paths(c, J.p, J.lanes, kOwnChunk));
+  std::vector<int> part(jobs.size());
+  for (int enough = 0; !enough;) {
+    double load[kStreams] = {};
+    size_t bytes[kStreams] = {};
+    for (size_t i = 0; i < jobs.size(); ++i) {
+      const Params& p = jobs[i].p;
+      const int h = int(std::min_element(load, load + parts) - load);
+      load[h] += double(p.width) * double(p.height) * double(p.spp) * double(p.bounces + 1);
+      part[i] = h;
+      bytes[h] = std::max(bytes[h], plans[i].bytes);
+    }
+    // workspaces before the first launch: to grow one waits for the device.
+    // Short of memory, fewer streams.
+    enough = 1;
+    for (int h = 0; h < parts && enough; ++h) {
+      const cudaError_t e = ws[h]->reserve(bytes[h]);
+      if (e == cudaSuccess) continue;
+      cudaGetLastError();
+      if (h == 0) { msg = cuda_msg("batch buffer allocation failed", e); return RM_ERR_ALLOC; }
+      parts = h;
+      enough = 0;
+    }
+  }
+  cudaError_t e = cudaSuccess;
+  if (parts > 1) e = cudaEventRecord(c->ev_fork, c->stream);
+  for (int h = 1; h < parts && e == cudaSuccess; ++h) e = cudaStreamWaitEvent(sts[h], c->ev_fork, 0);
+  for (size_t i = 0; i < jobs.size() && e == cudaSuccess; ++i) {
+    const BtJob& J = jobs[i];
+    const int h = part[i];
+    e = run_paths(c, J.s, J.p, J.lanes, J.seed, plans[i],
+                  PathsTarget{*ws[h], sts[h], J.hdr, J.rgb, J.dbg, RM_STAGE_BATCH, false});
+  }
+  for (int h = 1; h < parts; ++h) {
+    if (e == cudaSuccess) e = cudaEventRecord(c->ev_join[h - 1], sts[h]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_join[h - 1], 0);
+    else cudaStreamSynchronize(sts[h]);
+  }
+  if (e != cudaSuccess) { msg = cuda_msg("batch launch failed", e); return RM_ERR_CUDA; }
+  return RM_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -405,11 +492,13 @@ int rmcuda_render_batch(rmcuda_ctx* c, const rm_batch_item* items, int32_t n, ch
   cudaSetDevice(c->device);
   std::string msg;
   Prepared P;
-  int rc = prepare(c, items, n, c->batch.tuning.tile_shape, c->batch.tuning.bvh_width, P, msg);
+  int rc = prepare(c, items, n, c->batch.tuning.tile_shape, c->batch.tuning.bvh_width, false, P, msg);
   cudaEvent_t a = nullptr, b = nullptr;
   if (rc == RM_OK && c->profiling > 0 && cudaEventCreate(&a) == cudaSuccess && cudaEventCreate(&b) == cudaSuccess)
     cudaEventRecord(a, c->stream);
-  if (rc == RM_OK) rc = run_batch(c, P, c->batch.tuning, nullptr, msg);
+  c->batch.wave_log.clear();
+  if (rc == RM_OK) rc = run_own(c, P.own, msg);
+  if (rc == RM_OK && (P.own.empty() || !P.jobs.empty())) rc = run_batch(c, P, c->batch.tuning, nullptr, msg);
   if (a && b) {
     cudaEventRecord(b, c->stream);
     c->pending.push_back({RM_STAGE_BATCH, a, b});
@@ -447,7 +536,7 @@ int rmcuda_batch_tune(rmcuda_ctx* c, const rm_batch_item* items, int32_t n, rm_b
         const rm_batch_tuning t{pool, shape, scale, keep.graph_waves > 0 ? keep.graph_waves : 8, width};
         c->batch.tuning = t;
         Prepared P;
-        if ((rc = prepare(c, items, n, shape, width, P, msg)) != RM_OK) break;
+        if ((rc = prepare(c, items, n, shape, width, true, P, msg)) != RM_OK) break;
         if ((rc = run_batch(c, P, t, &win, msg)) != RM_OK) break;
         float ms = 0.f;
         cudaEventElapsedTime(&ms, win.t0, win.t1);
