@@ -156,6 +156,7 @@ struct rmcuda_ctx {
   bool hist_denoised = false;
   bool hist_had_history = false;  // the frame's temporal passes used the history before it
   rm_camera hist_prev_cam{};       // and this camera for reprojection
+  rmd::DevBuf gen;                 // k_restir_generate_tile's visibility rays
   rmd::DevBuf adj_scratch;         // the denoiser backward's intermediate images
   uint8_t* h_preview = nullptr;    // pinned RGB8 read-back of rmcuda_preview_last
   size_t h_preview_cap = 0;

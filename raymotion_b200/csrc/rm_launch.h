@@ -38,7 +38,11 @@ cudaError_t launch_paths(const Scene& s, const Params& p, uint64_t seed, const P
 // mode 0: every open pixel goes on, 1: those that fail the adaptive test, 2: none
 cudaError_t launch_paths_combine(const Params& p, const PathsArgs& a, int seg, int mode, int sms,
                                  cudaStream_t st);
-// stage 0 generate, 1 spatial (temporal + spatial reuse), 2 shade
+// K3; `scratch` holds restir_generate_scratch bytes
+size_t restir_generate_scratch(const Params& p, int sms);
+cudaError_t launch_restir_generate(const Scene& s, const Params& p, uint64_t seed, const GBufSoA& gb, const ResSoA& ri,
+                                   void* scratch, int sms, unsigned long long* ctr, uint32_t* err, cudaStream_t st);
+// stage 1 spatial (temporal + spatial reuse), 2 shade
 cudaError_t launch_restir_stage(int stage, const Scene& s, const Params& p, uint64_t seed, const GBufSoA& gb,
                                 const ResSoA& ri, const ResSoA& rm, const GBufSoA& hg, const ResSoA& hr, float* hdr,
                                 uint32_t* dbg, unsigned long long* ctr, uint32_t* err, cudaStream_t st);

@@ -738,6 +738,7 @@ int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_co
   const size_t npix = size_t(cfg.width) * size_t(cfg.height);
   cudaStream_t st = c->stream;
   cudaError_t e = ensure_frame(c, npix, pl.use_spatial);
+  if (e == cudaSuccess && pl.use_spatial) e = c->gen.reserve(restir_generate_scratch(p, c->sms));
   if (e != cudaSuccess) {
     msg = cuda_msg(pl.use_spatial ? "Metal ReSTIR buffer allocation failed" : "Metal image buffer allocation failed", e);
     return RM_ERR_ALLOC;
@@ -788,6 +789,9 @@ int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_co
         continue;
       }
       e = staged(c, RM_STAGE_GENERATE + stage, [&] {
+        if (stage == 0)
+          return launch_restir_generate(s, p, seed, c->gb.view(), c->rinit.view(), c->gen.ptr, c->sms,
+                                        ctr + 4 * RM_STAGE_GENERATE, err, st);
         return launch_restir_stage(stage, s, p, seed, c->gb.view(), c->rinit.view(), c->rmerged.view(), c->hg.view(),
                                    c->hres.view(), c->hdr.as<float>(), c->dbg.as<uint32_t>(),
                                    ctr + 4 * (RM_STAGE_GENERATE + stage), err, st);
@@ -898,7 +902,7 @@ void rmcuda_destroy(rmcuda_ctx* c) {
   c->sc.release();
   c->batch.release();
   for (DevBuf* b : {&c->hdr, &c->tmp_a, &c->tmp_b, &c->hist_col, &c->rgb, &c->dbg, &c->hash_out, &c->ctr, &c->err,
-                    &c->adj_scratch, &c->differ, &c->ctr_save, &c->paths})
+                    &c->adj_scratch, &c->gen, &c->differ, &c->ctr_save, &c->paths})
     b->release();
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   for (int h = 0; h < kStreams - 1; ++h) {
