@@ -827,7 +827,7 @@ def run_b200(args, world, rank, local):
     avg_s = ms_total / 1e3 / max(launches, 1)
     peak = measured_peaks()
     achieved = alg_bytes / avg_s / 1e9 if avg_s > 0 else 0.0
-    kernel_names = dict(plain="k_render_paths", shade="k_restir_shade", generate="k_restir_generate",
+    kernel_names = dict(plain="k_paths", shade="k_restir_shade", generate="k_restir_generate",
                         spatial="k_restir_spatial", temporal="k_denoise_temporal", atrous0="k_denoise_atrous",
                         atrous1="k_denoise_atrous", hash="k_hash", tonemap="k_tonemap",
                         wf_extend="k_wf_trace2" if merged_trace else "k_wf_extend",

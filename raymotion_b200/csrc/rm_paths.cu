@@ -33,19 +33,20 @@ namespace {
 
 using namespace wf;
 
-// Four 128-thread blocks per SM (128 registers, at most 72 bytes of spills in
-// opaque scenes): 1280x720, 16 spp, 150 k triangles 13.2 ms, at five blocks
-// (96 registers) 14.4, six 15.1, eight 14.3, three 14.6; as one thread per lane
-// and round (k_render_paths) 19.0.  At 64 spp 46.1 against 83.6; the Cornell box
-// at 320x180, 16 spp 1.13 against 2.19; 512x512, 32 spp, 200 k triangles 13.2
-// against 18.9.
+// Bound by the traversal's dependent node loads (long_scoreboard 3.4 of 8 cycles
+// between a warp's instructions, 8 of 32 lanes).  Four 128-thread blocks per SM
+// (128 registers): 1280x720, 16 spp, 150 k triangles 9.9 ms, at five (96
+// registers) 10.4, at six 9.7 with small frames slower; one thread per lane and
+// round (k_render_paths) 19.0, and this loop 13.2 before its two traversals
+// became one copy (Tracer::trace).  Cornell box at 320x180, 16 spp 1.0 against
+// 2.2 ms.
 //
-// Kept out: shadow and extension rays of different lanes in one traversal pass
+// Kept out, measured against 13.2: shadow and extension rays of different lanes in one traversal pass
 // (Cornell 2.0 ms, 512x512 18.1: each pass then shades half the lanes), a
 // lane's shadow ray and next extension ray one after the other in one loop (18
 // to 20 ms: the second ray's setup splits the warp).
 constexpr int kPathThreads = 128, kPathBlocks = 4;
-// Idle lanes of a warp that make it take new tasks: 16 (13.2 ms; 8: 14.3, 12:
+// Idle lanes of a warp that make it take new tasks: 16 (13.2 ms with two traversals; 8: 14.3, 12:
 // 13.6, 22: 13.2 and the Cornell box 1.17 against 1.13).
 constexpr int kRefill = 16;
 

@@ -635,8 +635,7 @@ PathsPlan plan_paths(rmcuda_ctx* c, const Params& p, int lanes, long long sample
   // When every lane has a thread of its own and the adaptive test cuts the
   // frame into segments, the one-launch lane kernel stays: its warps pass the
   // test without waiting for the slowest path of the frame (64x36, 256 spp, 2 k
-  // triangles 1.04 ms against 2.05; 128x72 3.10 against 3.13; 160x100 4.43
-  // against 4.02).
+  // triangles 1.77 ms against 2.21; 128x72 2.48 against 3.18).
   q.one_launch = segs > 1 && npix * lanes <= paths_one_wave(c->sms);
   if (q.one_launch) return q;
   const long long per_pixel = (long long)lanes * longest;
