@@ -867,13 +867,18 @@ cudaError_t run_adjoint(const Scene& s, const Params& p, uint64_t seed, const GB
   const size_t shmem = size_t(a.n_mat) * kMatParams * sizeof(float);
   a.use_shared = shmem <= 32 * 1024 ? 1 : 0;
   const size_t threads = size_t(p.width) * size_t(p.height) * size_t(a.lanes);
-  const unsigned grid = unsigned(std::min<size_t>(size_t(sms) * kAdjBlocks, (threads + kAdjThreads - 1) / kAdjThreads));
+  // fewer pixel lanes than the GPU's threads: narrower blocks, one on each SM
+  // (64x64, 2 spp 0.72 ms against 0.84, its ReSTIR frame 1.30 / 1.51, 130x97, 8
+  // spp 4.04 / 4.50)
+  const size_t per_sm = (threads + size_t(sms) * 32 - 1) / (size_t(sms) * 32) * 32;
+  const unsigned block = unsigned(std::min<size_t>(kAdjThreads, per_sm));
+  const unsigned grid = unsigned(std::min<size_t>(size_t(sms) * kAdjBlocks, (threads + block - 1) / block));
   const size_t sm = a.use_shared ? shmem : 0;
   const cudaError_t e = cudaMemsetAsync(a.next, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
-  if (!kRestir && !p.opaque) k_adjoint<1, false><<<grid, kAdjThreads, sm, st>>>(s, p, seed, gb, rm, a);
-  else if (p.restir_candidates > 1) k_adjoint<2, kRestir><<<grid, kAdjThreads, sm, st>>>(s, p, seed, gb, rm, a);
-  else k_adjoint<0, kRestir><<<grid, kAdjThreads, sm, st>>>(s, p, seed, gb, rm, a);
+  if (!kRestir && !p.opaque) k_adjoint<1, false><<<grid, block, sm, st>>>(s, p, seed, gb, rm, a);
+  else if (p.restir_candidates > 1) k_adjoint<2, kRestir><<<grid, block, sm, st>>>(s, p, seed, gb, rm, a);
+  else k_adjoint<0, kRestir><<<grid, block, sm, st>>>(s, p, seed, gb, rm, a);
   return cudaGetLastError();
 }
 
