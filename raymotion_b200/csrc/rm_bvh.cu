@@ -737,6 +737,7 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
     k_single_leaf<<<1, 1, 0, st>>>(d_tris, n, b.records.as<float4>(), b.parents.as<int>(), b.order.as<int>());
     RM_TRY(cudaGetLastError());
     b.max_depth = 1;
+    b.tree = true;
     RM_TRY(build_quads(b, st));
     return pack_tgeo(d_tris, b, st);
   }
@@ -789,6 +790,7 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(cudaMemcpyAsync(&b.max_depth, b.depth.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
   RM_TRY(cudaStreamSynchronize(st));
   if (b.max_depth > kStack) { err = "device BVH deeper than the traversal stack"; return cudaErrorInvalidValue; }
+  b.tree = true;
   RM_TRY(build_quads(b, st));
   return pack_tgeo(d_tris, b, st);
 }
@@ -1340,6 +1342,7 @@ cudaError_t build_ploc(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(cudaStreamSynchronize(st));
   if (b.max_depth > kStack) { err = "device BVH deeper than the traversal stack"; return cudaErrorInvalidValue; }
   b.n_records = n - 1;
+  b.tree = true;
   RM_TRY(build_quads(b, st));
   return pack_tgeo(d_tris, b, st);
 }
@@ -1388,6 +1391,7 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
     iv[2 + slot] = count;
   };
   int max_depth = 1;
+  bool tree = true;
   if (root_leaf) {
     put(0, 0, &nodes[0], nodes[0].offset, nodes[0].count);
     put(0, 1, nullptr, 0, -1);
@@ -1400,6 +1404,7 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
       for (int slot = 0; slot < 2; ++slot) {
         const int c = slot ? nodes[i].right : nodes[i].left;
         const rm_bvh_node& cn = nodes[c];
+        if (depth[size_t(c)] != 0) tree = false;  // another parent reached it before
         depth[size_t(c)] = depth[size_t(i)] + 1;
         max_depth = std::max(max_depth, depth[size_t(c)]);
         if (cn.count > 0) put(r, slot, &cn, cn.offset, cn.count);
@@ -1417,7 +1422,17 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
       }
   }
   if (max_depth > kStack) { err = "BVH deeper than 64 levels"; return false; }
+  if (!tree) {
+    // Shared subtrees are traversed once for each path to them: written out as
+    // a tree, the nodes must stay within the limit of a BVH without sharing (64
+    // levels that name one child twice would keep a ray busy for years).
+    std::vector<double> size(size_t(M), 1.0);
+    for (int i = M; i-- > 0;)
+      if (rec[size_t(i)] >= 0) size[size_t(i)] += size[size_t(nodes[i].left)] + size[size_t(nodes[i].right)];
+    if (size[0] >= double(kMaxLink)) { err = "BVH exceeds 16777215 nodes with its shared subtrees written out"; return false; }
+  }
   out.max_depth = max_depth;
+  out.tree = tree;
   out.n_records = n_rec;
   cudaError_t e;
   if ((e = out.records.reserve(recs.size() * sizeof(float))) != cudaSuccess ||

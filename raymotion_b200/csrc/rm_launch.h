@@ -254,6 +254,7 @@ struct DevBvh {
   int n_records = 0;
   int n_tris = 0;
   int max_depth = 0;
+  bool tree = true;  // every node of the records has one parent (a caller's BVH may share subtrees)
   // 4-wide BVH collapsed from the records (rm_quad.cu): 8 float4 per node;
   // qroots: nodes per level, then the binary record each node collapses
   DevBuf quads, qroots;

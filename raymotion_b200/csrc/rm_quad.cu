@@ -17,6 +17,10 @@
 // leaves.  The number of levels is at most the binary tree's depth, which the
 // host knows; a launch for an empty level ends at once.  The binary records
 // stay: a refit updates their boxes bottom-up and k_quad_refit copies them.
+//
+// That needs a tree: a subtree that several nodes of a caller's BVH share would
+// be written once for each path to it.  Such records become a node each, of
+// their two children (k_quad_pairs).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -130,6 +134,25 @@ __global__ void __launch_bounds__(128) k_quad_level(const float4* __restrict__ r
   }
 }
 
+// One node per record, of its two children: node and record share their index.
+__global__ void __launch_bounds__(128) k_quad_pairs(const float4* __restrict__ rec, int n_records, int* roots,
+                                                    int* level_n, int levels, float4* __restrict__ quads) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < levels) level_n[r] = r == 0 ? n_records : 0;  // (all in one level: what k_quad_refit sums)
+  if (r >= n_records) return;
+  roots[r] = r;
+  float4* q = quads + size_t(r) * 8;
+  const QChild a = read_child(rec, r, 0), b = read_child(rec, r, 1);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    q[2 * k] = make_float4(a.lo[k], b.lo[k], 0.0f, 0.0f);
+    q[2 * k + 1] = make_float4(a.hi[k], b.hi[k], 0.0f, 0.0f);
+  }
+  auto word = [](const QChild& c) { return c.cnt < 0 ? 0u : (uint32_t(c.cnt) << 24) | uint32_t(c.link); };
+  reinterpret_cast<uint4*>(q)[6] = make_uint4(word(a), word(b), 0u, 0u);
+  reinterpret_cast<int4*>(q)[7] = make_int4(a.cnt < 0 ? -1 : a.src, b.cnt < 0 ? -1 : b.src, -1, -1);
+}
+
 // Refit: each child's box copied from the (refitted) binary records, one
 // thread per child.
 __global__ void __launch_bounds__(256) k_quad_refit(const float4* __restrict__ rec, const int* __restrict__ level_n,
@@ -157,12 +180,18 @@ int quad_bound(int n_records) {
 
 cudaError_t build_quads(DevBvh& b, cudaStream_t st) {
   if (b.n_records <= 0) return cudaSuccess;
-  const int bound = quad_bound(b.n_records);
+  const int bound = b.tree ? quad_bound(b.n_records) : b.n_records;
   cudaError_t e;
   if ((e = b.quads.reserve(size_t(bound) * 8 * sizeof(float4))) != cudaSuccess) return e;
   if ((e = b.qroots.reserve((size_t(bound) + kStack + 2) * sizeof(int))) != cudaSuccess) return e;
   int* level_n = b.qroots.as<int>();
   int* roots = level_n + kStack + 2;
+  if (!b.tree) {
+    const int n = std::max(b.n_records, kStack + 2);
+    k_quad_pairs<<<(n + 127) / 128, 128, 0, st>>>(b.records.as<float4>(), b.n_records, roots, level_n, kStack + 2,
+                                                  b.quads.as<float4>());
+    return cudaGetLastError();
+  }
   const int levels = std::max(1, std::min(b.max_depth, kStack));
   k_quad_init<<<1, 128, 0, st>>>(roots, level_n, kStack + 2);
   long long most = 1;
@@ -176,7 +205,7 @@ cudaError_t build_quads(DevBvh& b, cudaStream_t st) {
 
 cudaError_t refit_quads(DevBvh& b, cudaStream_t st) {
   if (b.n_records <= 0) return cudaSuccess;
-  const long long n = 4ll * quad_bound(b.n_records);
+  const long long n = 4ll * (b.tree ? quad_bound(b.n_records) : b.n_records);
   const unsigned g = unsigned(std::min<long long>(148 * 8, (n + 255) / 256));
   k_quad_refit<<<g, 256, 0, st>>>(b.records.as<float4>(), b.qroots.as<int>(), kStack + 2, b.quads.as<float4>());
   return cudaGetLastError();

@@ -1,0 +1,93 @@
+"""Caller BVHs whose shape the 4-wide collapse (rm_quad.cu) cannot take as it
+takes a built one: subtrees that several nodes share.  Hits equal the oracle's
+bit for bit (they do not depend on the BVH); any-hit agrees."""
+import numpy as np
+import pytest
+
+from raymotion_b200 import RenderError, _abi
+
+from .gpu_util import random_rays
+from .test_gpu_quads import _check, _soup
+
+pytestmark = pytest.mark.gpu
+
+
+class Node:
+    """An inner node of two children, each a Node or a list of triangles; a
+    Node or list given to several parents is one node of the array."""
+
+    def __init__(self, left, right):
+        self.left, self.right = left, right
+
+
+def caller_bvh(sc, root, box=None):
+    """sc with the BVH of `root` as the caller's own: parents before their
+    children.  box(object, depth, mn, mx) may change a node's box."""
+    order, place = [], {}
+    todo = [(root, 1)]
+    depth = {}
+    while todo:  # a node's place: behind all of its parents'
+        t, d = todo.pop()
+        if depth.get(id(t), 0) >= d:
+            continue
+        depth[id(t)] = d
+        place[id(t)] = t
+        if isinstance(t, Node):
+            todo += [(t.left, d + 1), (t.right, d + 1)]
+    objects = sorted(place.values(), key=lambda t: depth[id(t)])
+    index = {id(t): i for i, t in enumerate(objects)}
+    bounds = {}
+    for t in reversed(objects):
+        if isinstance(t, Node):
+            a, b = bounds[id(t.left)], bounds[id(t.right)]
+            bounds[id(t)] = (np.minimum(a[0], b[0]), np.maximum(a[1], b[1]))
+        else:
+            v = np.concatenate([sc.tris[k][t] for k in ("v0", "v1", "v2")])
+            bounds[id(t)] = (v.min(0), v.max(0))
+    arr = np.zeros(len(objects), _abi.BVH_NODE_DTYPE)
+    for i, t in enumerate(objects):
+        mn, mx = bounds[id(t)]
+        if box:
+            mn, mx = box(t, depth[id(t)], mn, mx)
+        if isinstance(t, Node):
+            arr[i] = (tuple(mn), tuple(mx), index[id(t.left)], index[id(t.right)], 0, 0)
+        else:
+            arr[i] = (tuple(mn), tuple(mx), -1, -1, len(order), len(t))
+            order += t
+    assert sorted(order) == list(range(sc.n_tris))
+    return type(sc)(tris=sc.tris, light_tri=sc.light_tri, light_cdf=sc.light_cdf, light_total=sc.light_total,
+                    texels=sc.texels, verts64=sc.verts64, nodes=arr, bvh_tri=np.asarray(order, np.int32))
+
+
+def _twice(levels):
+    """A chain that names its next level as both children."""
+    t = Node([0], [1, 2])
+    for _ in range(levels):
+        t = Node(t, t)
+    return t
+
+
+def _two_parents():
+    a = Node([2], Node([3, 4], [5]))
+    return Node(Node([0], a), Node(Node([1], a), [6]))
+
+
+SHARED = {"child_twice": (3, lambda: _twice(1)), "chain": (3, lambda: _twice(8)), "two_parents": (7, _two_parents),
+          "shared_leaf": (2, lambda: (lambda a: Node(Node(a, [1]), a))([0]))}
+
+
+@pytest.mark.parametrize("shape", list(SHARED))
+def test_shared_subtrees(backend, oracle, shape):
+    n, root = SHARED[shape]
+    sc = oracle.with_reference_bvh(_soup(n, 31, spread=1.0))
+    backend.upload(caller_bvh(sc, root()), use_nodes=True)
+    rays = random_rays(4000, [-2, -2, -2], [2, 2, 2], n)
+    assert _check(backend, oracle, sc, rays) > 0.0
+
+
+def test_shared_subtrees_are_bounded(backend, oracle):
+    """Two to the 30 paths: refused on the host like any BVH of too many nodes."""
+    sc = oracle.with_reference_bvh(_soup(3, 31))
+    with pytest.raises(RenderError, match="shared subtrees") as e:
+        backend.upload(caller_bvh(sc, _twice(30)), use_nodes=True)
+    assert e.value.code == _abi.RM_ERR_BVH
