@@ -738,6 +738,7 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
     RM_TRY(cudaGetLastError());
     b.max_depth = 1;
     b.tree = true;
+    b.leaf_tris = n;
     RM_TRY(build_quads(b, st));
     return pack_tgeo(d_tris, b, st);
   }
@@ -791,6 +792,7 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(cudaStreamSynchronize(st));
   if (b.max_depth > kStack) { err = "device BVH deeper than the traversal stack"; return cudaErrorInvalidValue; }
   b.tree = true;
+  b.leaf_tris = n;
   RM_TRY(build_quads(b, st));
   return pack_tgeo(d_tris, b, st);
 }
@@ -1343,6 +1345,7 @@ cudaError_t build_ploc(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   if (b.max_depth > kStack) { err = "device BVH deeper than the traversal stack"; return cudaErrorInvalidValue; }
   b.n_records = n - 1;
   b.tree = true;
+  b.leaf_tris = n;
   RM_TRY(build_quads(b, st));
   return pack_tgeo(d_tris, b, st);
 }
@@ -1392,7 +1395,9 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
   };
   int max_depth = 1;
   bool tree = true;
+  long long leaf_tris = 0;
   if (root_leaf) {
+    leaf_tris = nodes[0].count;
     put(0, 0, &nodes[0], nodes[0].offset, nodes[0].count);
     put(0, 1, nullptr, 0, -1);
   } else {
@@ -1407,8 +1412,10 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
         if (depth[size_t(c)] != 0) tree = false;  // another parent reached it before
         depth[size_t(c)] = depth[size_t(i)] + 1;
         max_depth = std::max(max_depth, depth[size_t(c)]);
-        if (cn.count > 0) put(r, slot, &cn, cn.offset, cn.count);
-        else {
+        if (cn.count > 0) {
+          put(r, slot, &cn, cn.offset, cn.count);
+          leaf_tris += cn.count;
+        } else {
           put(r, slot, &cn, rec[size_t(c)], 0);
           parents[size_t(rec[size_t(c)])] = (r << 1) | slot;
         }
@@ -1433,6 +1440,7 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
   }
   out.max_depth = max_depth;
   out.tree = tree;
+  out.leaf_tris = leaf_tris;
   out.n_records = n_rec;
   cudaError_t e;
   if ((e = out.records.reserve(recs.size() * sizeof(float))) != cudaSuccess ||

@@ -255,6 +255,7 @@ struct DevBvh {
   int n_tris = 0;
   int max_depth = 0;
   bool tree = true;  // every node of the records has one parent (a caller's BVH may share subtrees)
+  long long leaf_tris = 0;  // triangles of all leaves (a caller's leaves may overlap or leave some out)
   // 4-wide BVH collapsed from the records (rm_quad.cu): 8 float4 per node;
   // qroots: nodes per level, then the binary record each node collapses
   DevBuf quads, qroots;
@@ -286,7 +287,8 @@ cudaError_t build_quads(DevBvh& bvh, cudaStream_t st);
 cudaError_t refit_quads(DevBvh& bvh, cudaStream_t st);
 // Collapse the binary records into the 8-wide compressed BVH (rm_wide.cu).
 // Leaves n_wide at 0 (the binary BVH stays in use) when a node cannot be
-// encoded or the wide tree would be deeper than the traversal stack.
+// encoded, the wide tree would be deeper than the traversal stack, or the
+// records are no tree whose leaves hold each triangle once.
 cudaError_t build_wide(DevBvh& bvh, cudaStream_t st);
 // Caller-provided scratch of an LBVH build (device pointers; see rm_noalloc.cu).
 struct LbvhScratch {

@@ -206,6 +206,8 @@ cudaError_t build_wide(DevBvh& b, cudaStream_t st) {
   b.n_wide = 0;
   if (b.n_records <= 0 || b.n_tris <= 0) return cudaSuccess;
   const int n = b.n_tris;
+  // the buffers below hold each record and each triangle once
+  if (!b.tree || b.leaf_tris != n) return cudaSuccess;
   // at most one wide node per binary record, one frontier item per wide node
   cudaError_t e;
   if ((e = b.wnodes.reserve(size_t(b.n_records) * 5 * sizeof(float4))) != cudaSuccess) return e;

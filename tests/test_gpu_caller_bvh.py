@@ -1,5 +1,5 @@
-"""Caller BVHs whose shape the 4-wide collapse (rm_quad.cu) cannot take as it
-takes a built one: subtrees that several nodes share.  Hits equal the oracle's
+"""Caller BVHs whose shape the collapses (rm_quad.cu, rm_wide.cu) cannot take as
+they take a built one: subtrees that several nodes share, leaves that overlap.  Hits equal the oracle's
 bit for bit (they do not depend on the BVH); any-hit agrees."""
 import numpy as np
 import pytest
@@ -76,8 +76,11 @@ SHARED = {"child_twice": (3, lambda: _twice(1)), "chain": (3, lambda: _twice(8))
           "shared_leaf": (2, lambda: (lambda a: Node(Node(a, [1]), a))([0]))}
 
 
+@pytest.mark.parametrize("wide", [False, True], ids=["default", "wide"])
 @pytest.mark.parametrize("shape", list(SHARED))
-def test_shared_subtrees(backend, oracle, shape):
+def test_shared_subtrees(backend, oracle, shape, wide, monkeypatch):
+    if wide:
+        monkeypatch.setenv("RAYMOTION_CUDA_WIDE", "1")
     n, root = SHARED[shape]
     sc = oracle.with_reference_bvh(_soup(n, 31, spread=1.0))
     backend.upload(caller_bvh(sc, root()), use_nodes=True)
@@ -91,3 +94,19 @@ def test_shared_subtrees_are_bounded(backend, oracle):
     with pytest.raises(RenderError, match="shared subtrees") as e:
         backend.upload(caller_bvh(sc, _twice(30)), use_nodes=True)
     assert e.value.code == _abi.RM_ERR_BVH
+
+
+def test_overlapping_leaves_in_the_wide_bvh(backend, oracle, monkeypatch):
+    """Two leaves over one range of triangles: more triangles in leaves than the scene has."""
+    monkeypatch.setenv("RAYMOTION_CUDA_WIDE", "1")
+    sc = oracle.with_reference_bvh(_soup(8, 32, spread=1.0))
+    caller = caller_bvh(sc, Node(Node([0, 1, 2], [3, 4]), Node([5], [6, 7])))
+    leaf = [i for i in range(len(caller.nodes)) if caller.nodes["count"][i] > 0]
+    for i in leaf:  # every leaf: the first four positions, or the last four
+        caller.nodes[i]["count"], caller.nodes[i]["offset"] = 4, 0 if i in leaf[:2] else 4
+        caller.nodes[i]["mn"], caller.nodes[i]["mx"] = caller.nodes[0]["mn"], caller.nodes[0]["mx"]
+    for i in set(range(len(caller.nodes))) - set(leaf):
+        caller.nodes[i]["mn"], caller.nodes[i]["mx"] = caller.nodes[0]["mn"], caller.nodes[0]["mx"]
+    backend.upload(caller, use_nodes=True)
+    rays = random_rays(4000, [-2, -2, -2], [2, 2, 2], 8)
+    assert _check(backend, oracle, sc, rays) > 0.0
