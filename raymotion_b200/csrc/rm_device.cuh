@@ -396,7 +396,9 @@ struct Trav {
 // Box test: Trav's, with the near and far bounds picked by the sign of i when
 // the node is read (near is lo for i >= 0) instead of by min / max; an axis
 // whose o i overflows culls nothing, as there.
-constexpr int kQuadStack = 3 * kStack / 2 + 4;  // at most three pushed per two binary levels
+// A node on the way pushes three subtrees at most and lies one binary level or
+// more below the one before it (its children may include one it never opened).
+constexpr int kQuadStack = 3 * kStack + 4;
 
 struct QTrav {
   float ox, oy, oz, dx, dy, dz, ix, iy, iz;

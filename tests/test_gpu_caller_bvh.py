@@ -110,3 +110,34 @@ def test_overlapping_leaves_in_the_wide_bvh(backend, oracle, monkeypatch):
     backend.upload(caller, use_nodes=True)
     rays = random_rays(4000, [-2, -2, -2], [2, 2, 2], 8)
     assert _check(backend, oracle, sc, rays) > 0.0
+
+
+def test_most_subtrees_pending(backend, oracle):
+    """64 levels whose every node holds the rest of the chain and a larger subtree
+    of three leaves: the collapse opens that subtree twice, so that each 4-wide
+    node pushes three subtrees and the chain goes on one level further down.  All
+    boxes hold the rays' origins and the chain is entered first."""
+    inner = 62  # (the leaves of the last subtree are on level 64)
+    n = 3 * (inner - 1) + 2
+    sc = oracle.with_reference_bvh(_soup(n, 33, spread=1.0))
+    tri = iter(range(n))
+    rest, size, half = Node([next(tri)], [next(tri)]), {}, 4.0
+    size[id(rest)] = half
+    for _ in range(inner - 1):
+        half /= 0.98
+        pair = Node([next(tri)], [next(tri)])
+        three = Node([next(tri)], pair)
+        rest = Node(rest, three)
+        size.update({id(pair): 0.99 * half, id(three): half, id(rest): half})
+    assert next(tri, None) is None
+
+    def box(t, depth, mn, mx):
+        h = size.get(id(t), 3.9)  # (a leaf holds the origins too)
+        assert (mn > -h).all() and (mx < h).all()
+        return np.full(3, -h, np.float32), np.full(3, h, np.float32)
+
+    builds = backend.stats()["bvh_builds"]
+    backend.upload(caller_bvh(sc, rest, box), use_nodes=True)
+    assert backend.stats()["bvh_builds"] == builds  # not too deep for the caller's BVH
+    rays = random_rays(4000, [-1.5] * 3, [1.5] * 3, 34)
+    assert _check(backend, oracle, sc, rays) > 0.05
