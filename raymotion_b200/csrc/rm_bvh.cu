@@ -1394,7 +1394,14 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
     iv[2 + slot] = count;
   };
   int max_depth = 1;
-  bool tree = true;
+  bool shared = false, nested = true;  // (the root's own box is not tested)
+  auto ordered_box = [](const rm_bvh_node& c) {
+    return c.mn.x <= c.mx.x && c.mn.y <= c.mx.y && c.mn.z <= c.mx.z;
+  };
+  auto inside = [](const rm_bvh_node& c, const rm_bvh_node& p) {
+    return p.mn.x <= c.mn.x && p.mn.y <= c.mn.y && p.mn.z <= c.mn.z && c.mx.x <= p.mx.x && c.mx.y <= p.mx.y &&
+           c.mx.z <= p.mx.z;
+  };
   long long leaf_tris = 0;
   if (root_leaf) {
     leaf_tris = nodes[0].count;
@@ -1409,7 +1416,8 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
       for (int slot = 0; slot < 2; ++slot) {
         const int c = slot ? nodes[i].right : nodes[i].left;
         const rm_bvh_node& cn = nodes[c];
-        if (depth[size_t(c)] != 0) tree = false;  // another parent reached it before
+        if (depth[size_t(c)] != 0) shared = true;  // another parent reached it before
+        if (!(ordered_box(cn) && (i == 0 || inside(cn, nodes[i])))) nested = false;
         depth[size_t(c)] = depth[size_t(i)] + 1;
         max_depth = std::max(max_depth, depth[size_t(c)]);
         if (cn.count > 0) {
@@ -1429,7 +1437,7 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
       }
   }
   if (max_depth > kStack) { err = "BVH deeper than 64 levels"; return false; }
-  if (!tree) {
+  if (shared) {
     // Shared subtrees are traversed once for each path to them: written out as
     // a tree, the nodes must stay within the limit of a BVH without sharing (64
     // levels that name one child twice would keep a ray busy for years).
@@ -1439,7 +1447,7 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
     if (size[0] >= double(kMaxLink)) { err = "BVH exceeds 16777215 nodes with its shared subtrees written out"; return false; }
   }
   out.max_depth = max_depth;
-  out.tree = tree;
+  out.tree = !shared && nested;
   out.leaf_tris = leaf_tris;
   out.n_records = n_rec;
   cudaError_t e;

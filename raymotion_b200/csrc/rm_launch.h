@@ -254,7 +254,9 @@ struct DevBvh {
   int n_records = 0;
   int n_tris = 0;
   int max_depth = 0;
-  bool tree = true;  // every node of the records has one parent (a caller's BVH may share subtrees)
+  // The records may be collapsed: every node has one parent, and its box is
+  // ordered and inside its parent's (a caller's BVH may break either).
+  bool tree = true;
   long long leaf_tris = 0;  // triangles of all leaves (a caller's leaves may overlap or leave some out)
   // 4-wide BVH collapsed from the records (rm_quad.cu): 8 float4 per node;
   // qroots: nodes per level, then the binary record each node collapses

@@ -18,9 +18,10 @@
 // host knows; a launch for an empty level ends at once.  The binary records
 // stay: a refit updates their boxes bottom-up and k_quad_refit copies them.
 //
-// That needs a tree: a subtree that several nodes of a caller's BVH share would
-// be written once for each path to it.  Such records become a node each, of
-// their two children (k_quad_pairs).
+// That needs a tree of nested boxes.  A subtree that several nodes of a caller's
+// BVH share would be written once for each path to it, and the box of an opened
+// child is not tested, which hides subtrees whose boxes reach out of it.  Such
+// records become a node each, of their two children (k_quad_pairs).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -143,10 +144,11 @@ __global__ void __launch_bounds__(128) k_quad_pairs(const float4* __restrict__ r
   roots[r] = r;
   float4* q = quads + size_t(r) * 8;
   const QChild a = read_child(rec, r, 0), b = read_child(rec, r, 1);
+  // a box's bounds may come in either order: the test takes the lesser as near
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    q[2 * k] = make_float4(a.lo[k], b.lo[k], 0.0f, 0.0f);
-    q[2 * k + 1] = make_float4(a.hi[k], b.hi[k], 0.0f, 0.0f);
+    q[2 * k] = make_float4(fminf(a.lo[k], a.hi[k]), fminf(b.lo[k], b.hi[k]), 0.0f, 0.0f);
+    q[2 * k + 1] = make_float4(fmaxf(a.lo[k], a.hi[k]), fmaxf(b.lo[k], b.hi[k]), 0.0f, 0.0f);
   }
   auto word = [](const QChild& c) { return c.cnt < 0 ? 0u : (uint32_t(c.cnt) << 24) | uint32_t(c.link); };
   reinterpret_cast<uint4*>(q)[6] = make_uint4(word(a), word(b), 0u, 0u);

@@ -1,5 +1,6 @@
 """Caller BVHs whose shape the collapses (rm_quad.cu, rm_wide.cu) cannot take as
-they take a built one: subtrees that several nodes share, leaves that overlap.  Hits equal the oracle's
+they take a built one: subtrees that several nodes share, leaves that overlap,
+boxes that do not hold their children's or have their bounds swapped.  Hits equal the oracle's
 bit for bit (they do not depend on the BVH); any-hit agrees."""
 import numpy as np
 import pytest
@@ -7,7 +8,7 @@ import pytest
 from raymotion_b200 import RenderError, _abi
 
 from .gpu_util import random_rays
-from .test_gpu_quads import _check, _soup
+from .test_gpu_quads import _check, _soup, _trace
 
 pytestmark = pytest.mark.gpu
 
@@ -141,3 +142,37 @@ def test_most_subtrees_pending(backend, oracle):
     assert backend.stats()["bvh_builds"] == builds  # not too deep for the caller's BVH
     rays = random_rays(4000, [-1.5] * 3, [1.5] * 3, 34)
     assert _check(backend, oracle, sc, rays) > 0.05
+
+
+@pytest.mark.parametrize("wide", [False, True], ids=["default", "wide"])
+@pytest.mark.parametrize("what", ["too_small", "swapped_inner", "swapped_leaf", "swapped_one_axis"])
+def test_boxes_are_taken_as_given(backend, oracle, what, wide, monkeypatch):
+    """A subtree is entered through every box on its way, as the reference enters
+    it, also where an inner box misses part of it or gives its bounds the other
+    way round; the oracle walks the same nodes."""
+    if wide:
+        monkeypatch.setenv("RAYMOTION_CUDA_WIDE", "1")
+    sc = oracle.with_reference_bvh(_soup(200, 35))
+    nodes = sc.nodes.copy()
+    inner = nodes["count"] == 0
+    pick = {"too_small": inner, "swapped_inner": inner}.get(what, ~inner)
+    pick = np.flatnonzero(pick)[1::3]
+    mn, mx = nodes["mn"].copy(), nodes["mx"].copy()
+    if what == "too_small":
+        nodes["mn"][pick], nodes["mx"][pick] = mn[pick] + 0.3 * (mx - mn)[pick], mx[pick] - 0.3 * (mx - mn)[pick]
+    else:
+        axes = [1] if what == "swapped_one_axis" else [0, 1, 2]
+        for a in axes:
+            nodes["mn"][pick, a], nodes["mx"][pick, a] = mx[pick, a], mn[pick, a]
+    caller = type(sc)(tris=sc.tris, light_tri=sc.light_tri, light_cdf=sc.light_cdf, light_total=sc.light_total,
+                      texels=sc.texels, verts64=sc.verts64, nodes=nodes, bvh_tri=sc.bvh_tri)
+    backend.upload(caller, use_nodes=True)
+    rays = random_rays(8000, [-3, -3, -3], [3, 3, 3], 36)
+    every = (oracle.trace(sc, rays)[0] >= 0).mean()
+    if what == "too_small":
+        # (which hit is the closest of those found depends on the order of the visits)
+        hit = oracle.trace(caller, rays, any_hit=True)[0] >= 0
+        assert np.array_equal(_trace(backend, rays, any_hit=True)[0] >= 0, hit)
+        assert 0 < hit.mean() < every
+    else:
+        assert _check(backend, oracle, caller, rays) == every
