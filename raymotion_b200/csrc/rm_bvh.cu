@@ -1096,14 +1096,17 @@ struct PlocSmall {
 __global__ void __launch_bounds__(1024) k_ploc_small(const int* __restrict__ cl0, const int* __restrict__ cl1,
                                                      PlocState* st, float4* __restrict__ blo,
                                                      float4* __restrict__ bhi, int2* __restrict__ child,
-                                                     int n_leaves) {
+                                                     int n_leaves, int* left) {
   extern __shared__ __align__(16) unsigned char ploc_small[];
   PlocSmall& sh = *reinterpret_cast<PlocSmall*>(ploc_small);
   __shared__ int2 warp_sum[32];
   const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
   int C = st->clusters, next = st->next_node;
   bool force = st->force != 0;
-  if (C > kPlocSmall) return;  // not reached yet
+  if (C > kPlocSmall) {  // not reached yet
+    if (tid == 0) *left = C;
+    return;
+  }
   const int* cl = st->side ? cl1 : cl0;
   for (int i = tid; i < C; i += 1024) {
     const int c = cl[i];
@@ -1165,23 +1168,20 @@ __global__ void __launch_bounds__(1024) k_ploc_small(const int* __restrict__ cl0
     }
     __syncthreads();
   }
-  if (tid == 0) {
-    st->clusters = C;
-    st->next_node = next;
-  }
+  if (tid == 0) *left = C;
 }
 
 // Leaf position in depth-first order and depth: walk to the root adding the
-// sizes of left siblings.  Only the n leaves walk; max depth -> *depth.
+// sizes of left siblings.  Only the n leaves walk; max depth -> *depth.  The
+// layout kernels leave an unfinished tree (*left clusters, not one) alone.
 __global__ void k_ploc_layout(int n, int root, const float4* __restrict__ blo, const float4* __restrict__ bhi,
                               const int2* __restrict__ child, const int* __restrict__ order, int* __restrict__ pos,
-                              int* __restrict__ out_order, int* __restrict__ depth) {
+                              int* __restrict__ out_order, const int* __restrict__ left, int* __restrict__ depth) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || *left != 1) return;
   int off = 0, d = 1, cur = i;
   while (cur != root) {
     const int p = __float_as_int(bhi[cur].w);
-    if (p < n) break;  // no parent: an unfinished tree
     const int2 c = child[p - n];
     if (c.y == cur) off += __float_as_int(blo[c.x].w);
     cur = p;
@@ -1198,13 +1198,13 @@ __global__ void k_ploc_layout(int n, int root, const float4* __restrict__ blo, c
 // sibling's subtree on the way up (a subtree of s leaves has s - 1).  The
 // nearer child of a descent then usually sits in the next record.
 __global__ void k_ploc_preorder(int n, int root, const float4* __restrict__ blo, const float4* __restrict__ bhi,
-                                const int2* __restrict__ child, int* __restrict__ pre) {
+                                const int2* __restrict__ child, const int* __restrict__ left,
+                                int* __restrict__ pre) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;  // internal node n + k
-  if (k >= n - 1) return;
+  if (k >= n - 1 || *left != 1) return;
   int off = 0, d = 0, cur = n + k;
   while (cur != root) {
     const int p = __float_as_int(bhi[cur].w);
-    if (p < n) break;  // no parent: an unfinished tree
     const int2 c = child[p - n];
     off += 1;
     if (c.y == cur) off += __float_as_int(blo[c.x].w) - 1;
@@ -1222,9 +1222,9 @@ __device__ __forceinline__ int ploc_first(int node, int n, const int2* __restric
 
 __global__ void k_ploc_emit(int n, int leaf_max, const float4* __restrict__ blo, const float4* __restrict__ bhi,
                             const int2* __restrict__ child, const int* __restrict__ pos, const int* __restrict__ pre,
-                            float4* recs, int* parents) {
+                            const int* __restrict__ left, float4* recs, int* parents) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;  // internal node n + k
-  if (k >= n - 1) return;
+  if (k >= n - 1 || *left != 1) return;
   const int node = n + k;
   const int rec_id = pre[k];
   float4* rec = recs + size_t(rec_id) * 4;
@@ -1295,7 +1295,7 @@ cudaError_t build_ploc(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(b.knodes.reserve(size_t(n) * sizeof(int2)));
   RM_TRY(b.ranges.reserve(size_t(n) * 3 * sizeof(int) + sizeof(int) + size_t(tiles) * sizeof(int2) + sizeof(PlocState)));
   RM_TRY(b.kcount.reserve(size_t(n) * sizeof(int)));
-  RM_TRY(b.depth.reserve(sizeof(int)));
+  RM_TRY(b.depth.reserve(2 * sizeof(int)));
   float4* blo = b.kbox.as<float4>();
   float4* bhi = blo + total;
   int2* child = b.knodes.as<int2>();
@@ -1324,24 +1324,27 @@ cudaError_t build_ploc(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
     RM_TRY(cudaMemcpyAsync(&C, &state->clusters, sizeof(int), cudaMemcpyDeviceToHost, st));
     RM_TRY(cudaStreamSynchronize(st));
   }
-  k_ploc_small<<<1, 1024, sizeof(PlocSmall), st>>>(cl0, cl1, state, blo, bhi, child, n);
+  int* depth = b.depth.as<int>();  // the tree's depth, then the clusters left
+  k_ploc_small<<<1, 1024, sizeof(PlocSmall), st>>>(cl0, cl1, state, blo, bhi, child, n, depth + 1);
   RM_TRY(cudaGetLastError());
   const int root = total - 1;
-  // layout (of a complete tree: an unfinished one, whose root is missing, ends the walks at their bound)
   int* pos = b.kcount.as<int>();
-  RM_TRY(cudaMemsetAsync(b.depth.ptr, 0, sizeof(int), st));
-  k_ploc_layout<<<(n + 255) / 256, 256, 0, st>>>(n, root, blo, bhi, child, sorted, pos, b.order.as<int>(),
-                                                 b.depth.as<int>());
+  RM_TRY(cudaMemsetAsync(depth, 0, sizeof(int), st));
+  k_ploc_layout<<<(n + 255) / 256, 256, 0, st>>>(n, root, blo, bhi, child, sorted, pos, b.order.as<int>(), depth + 1,
+                                                 depth);
   int* pre = pair;  // the cluster arrays are free once the tree is built
-  k_ploc_preorder<<<(n - 1 + 255) / 256, 256, 0, st>>>(n, root, blo, bhi, child, pre);
+  k_ploc_preorder<<<(n - 1 + 255) / 256, 256, 0, st>>>(n, root, blo, bhi, child, depth + 1, pre);
   RM_TRY(b.records.reserve(size_t(n - 1) * 4 * sizeof(float4)));
   RM_TRY(b.parents.reserve(size_t(n - 1) * sizeof(int)));
   RM_TRY(b.counters.reserve(size_t(n - 1) * sizeof(int)));
-  k_ploc_emit<<<(n - 1 + 255) / 256, 256, 0, st>>>(n, leaf_max, blo, bhi, child, pos, pre, b.records.as<float4>(),
-                                                   b.parents.as<int>());
+  k_ploc_emit<<<(n - 1 + 255) / 256, 256, 0, st>>>(n, leaf_max, blo, bhi, child, pos, pre, depth + 1,
+                                                   b.records.as<float4>(), b.parents.as<int>());
   RM_TRY(cudaGetLastError());
-  RM_TRY(cudaMemcpyAsync(&b.max_depth, b.depth.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  int built[2] = {0, 0};
+  RM_TRY(cudaMemcpyAsync(built, depth, sizeof(built), cudaMemcpyDeviceToHost, st));
   RM_TRY(cudaStreamSynchronize(st));
+  if (built[1] != 1) { err = "clustering build produced a malformed tree"; return cudaErrorInvalidValue; }
+  b.max_depth = built[0];
   if (b.max_depth > kStack) { err = "device BVH deeper than the traversal stack"; return cudaErrorInvalidValue; }
   b.n_records = n - 1;
   b.tree = true;
