@@ -703,14 +703,13 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks) k_adjoint(Scene s, Pa
       if (kRestir && indirect) {
         const Primary q = primary(gb, id);
         const HeldLight h = held_light(p, rm, id, q);
-        bool early = !again;
         float nx2 = b0x, ny2 = b0y, nz2 = b0z;
         int pdelta = 0;
         Bsdf e0{0.f, 0.f, 0.f, 0.f};
         if (again) pt.rng.state = start_state;
         while (si < p.spp) {
           if (!again) start_state = pt.rng.state;
-          early = false;
+          bool early = false;
           if (pt.U() < q.spec_prob) {
             float hx, hy, hz;
             pt.sample_ggx_half(q.alpha2, q.nx, q.ny, q.nz, hx, hy, hz);

@@ -885,14 +885,14 @@ struct PlocState {
   int force;      // the last round merged nothing: merge neighbours (0,1), (2,3), ...
   int side;       // which cluster list is current
   // the round being applied
-  int in_clusters, in_force, in_side, in_next, merge;
+  int in_clusters, in_side, in_next, merge;
   unsigned int done;  // blocks of k_ploc_round that have counted
 };
 
 __global__ void k_ploc_leaves(const rm_triangle* __restrict__ tris, const int* __restrict__ order, int n,
                               float4* __restrict__ blo, float4* __restrict__ bhi, int* __restrict__ cl, PlocState* state) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *state = PlocState{n, n, 0, 0, 0, 0, 0, 0, 0, 0u};
+  if (i == 0) *state = PlocState{n, n, 0, 0, 0, 0, 0, 0, 0u};
   if (i >= n) return;
   const Box b = tri_box(tris[order[i]]);
   blo[i] = make_float4(b.mn[0], b.mn[1], b.mn[2], __int_as_float(1));
@@ -1024,7 +1024,6 @@ __global__ void __launch_bounds__(kPlocTile) k_ploc_round(const int* __restrict_
   }
   if (threadIdx.x == 0) {
     st->in_clusters = C;
-    st->in_force = force;
     st->in_side = st->side;
     st->in_next = st->next_node;
     st->merge = carry.x > 0 ? 1 : 0;
