@@ -283,8 +283,16 @@ struct PathsTarget {
   int stage;   // whose counters the image's work adds to
   bool timed;  // by the profiler, on the context stream
 };
-// `samples`: the most whose values the workspace holds.
-PathsPlan plan_paths(rmcuda_ctx* c, const rmd::Params& p, int lanes, long long samples);
+// What a workspace may take: the most samples whose values it holds; bare: none
+// for several lanes per pixel.
+struct PathsRoom {
+  long long samples;
+  bool bare = false;
+};
+// The next smaller room, for a workspace that the device had no memory for;
+// false when there is none.
+bool smaller_paths(rmcuda_ctx* c, PathsRoom& r);
+PathsPlan plan_paths(rmcuda_ctx* c, const rmd::Params& p, int lanes, const PathsRoom& r);
 // The plain chain of one image (rm_paths.cu), enqueued on t.stream.
 cudaError_t run_paths(rmcuda_ctx* c, const rmd::Scene& s, const rmd::Params& p, int lanes, uint64_t seed,
                       const PathsPlan& q, const PathsTarget& t);

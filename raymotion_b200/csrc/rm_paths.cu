@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kPathThreads, kPathBlocks) k_paths(Scene s, Pa
         n = 0;
         sr = sg = sb = sum_l = sum_l2 = 0.0f;
         active = fresh = si < p.spp;
-        if (!active) a.state[slot] = pt.rng.state;
+        if (L > 1 && !active) a.state[slot] = pt.rng.state;
       }
     }
     if (!__any_sync(full, active)) {

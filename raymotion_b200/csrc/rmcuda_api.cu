@@ -611,11 +611,13 @@ cudaError_t ensure_frame(rmcuda_ctx* c, size_t npix, bool restir) {
 
 // The plain chain of one image (rm_paths.cu): chunks of at most kPathChunk
 // samples (their values take 16 bytes each), each in segments that end where
-// the adaptive test applies.
+// the adaptive test applies.  Where the device has not that much memory left,
+// smaller chunks do (down to one wave of lanes), and in the end the lane kernels,
+// which need none.
 constexpr long long kPathChunk = 16ll << 20;
 constexpr int kPathSamples = 4096;  // most samples of a pixel in one segment
 
-PathsPlan plan_paths(rmcuda_ctx* c, const Params& p, int lanes, long long samples) {
+static PathsPlan plan_paths(rmcuda_ctx* c, const Params& p, int lanes, long long samples) {
   PathsPlan q;
   const long long npix = (long long)p.width * p.height;
   const int rounds = (p.spp + lanes - 1) / lanes;
@@ -648,12 +650,28 @@ PathsPlan plan_paths(rmcuda_ctx* c, const Params& p, int lanes, long long sample
   };
   const size_t px = size_t(q.chunk), several = lanes > 1 ? 1 : 0, multi = segs > 1 ? several : 0;
   q.val = take(several * px * size_t(per_pixel) * sizeof(float4));
-  q.state = take(px * size_t(lanes) * sizeof(uint32_t));
+  q.state = take(several * px * size_t(lanes) * sizeof(uint32_t));
   q.gsum = take(multi * px * sizeof(float4));
   q.gsl2 = take(multi * px * sizeof(float));
   q.list[0] = take(multi * px * sizeof(int));
   q.list[1] = take(multi * px * sizeof(int));
   q.counts = take((segs + 1) * 2 * sizeof(int));
+  return q;
+}
+
+bool smaller_paths(rmcuda_ctx* c, PathsRoom& r) {
+  if (r.bare) return false;
+  if (r.samples / 4 >= paths_one_wave(c->sms)) r.samples /= 4;
+  else r.bare = true;
+  return true;
+}
+
+PathsPlan plan_paths(rmcuda_ctx* c, const Params& p, int lanes, const PathsRoom& r) {
+  PathsPlan q = plan_paths(c, p, lanes, r.samples);
+  if (r.bare && lanes > 1) {
+    q.one_launch = true;
+    q.bytes = 0;
+  }
   return q;
 }
 
@@ -747,7 +765,17 @@ int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_co
   uint32_t* err = c->err.as<uint32_t>();
   if (!pl.use_spatial) {
     c->last_chain = pl.lanes;
-    e = run_paths(c, s, p, pl.lanes, seed, plan_paths(c, p, pl.lanes, kPathChunk),
+    PathsRoom room{kPathChunk};
+    PathsPlan q = plan_paths(c, p, pl.lanes, room);
+    while (q.bytes && (e = c->paths.reserve(q.bytes)) != cudaSuccess) {
+      cudaGetLastError();
+      if (!smaller_paths(c, room)) {
+        msg = cuda_msg("Metal image buffer allocation failed", e);
+        return RM_ERR_ALLOC;
+      }
+      q = plan_paths(c, p, pl.lanes, room);
+    }
+    e = run_paths(c, s, p, pl.lanes, seed, q,
                   PathsTarget{c->paths, st, c->hdr.as<float>(), d_rgb, c->dbg.as<uint32_t>(), RM_STAGE_PLAIN, true});
     if (e != cudaSuccess) { msg = cuda_msg("render_paths launch failed", e); return RM_ERR_CUDA; }
     c->last_final = c->hdr.as<float>();

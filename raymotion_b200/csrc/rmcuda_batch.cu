@@ -384,29 +384,34 @@ int run_own(rmcuda_ctx* c, const std::vector<BtJob>& jobs, std::string& msg) {
     sts[h] = h == 0 ? c->stream : c->side_stream[h - 1];
     ws[h] = h == 0 ? &c->paths : &c->batch.paths[h - 1];
   }
-  std::vector<PathsPlan> plans;
-  for (const BtJob& J : jobs) plans.push_back(plan_paths(c, J.p, J.lanes, kOwnChunk));
+  std::vector<PathsPlan> plans(jobs.size());
   std::vector<int> part(jobs.size());
-  for (int enough = 0; !enough;) {
+  PathsRoom room{kOwnChunk};
+  for (bool enough = false; !enough;) {
     double load[kStreams] = {};
     size_t bytes[kStreams] = {};
     for (size_t i = 0; i < jobs.size(); ++i) {
       const Params& p = jobs[i].p;
+      plans[i] = plan_paths(c, p, jobs[i].lanes, room);
       const int h = int(std::min_element(load, load + parts) - load);
       load[h] += double(p.width) * double(p.height) * double(p.spp) * double(p.bounces + 1);
       part[i] = h;
       bytes[h] = std::max(bytes[h], plans[i].bytes);
     }
     // workspaces before the first launch: to grow one waits for the device.
-    // Short of memory, fewer streams.
-    enough = 1;
+    // Short of memory, fewer streams, then smaller chunks.
+    enough = true;
     for (int h = 0; h < parts && enough; ++h) {
-      const cudaError_t e = ws[h]->reserve(bytes[h]);
+      const cudaError_t e = bytes[h] ? ws[h]->reserve(bytes[h]) : cudaSuccess;
       if (e == cudaSuccess) continue;
       cudaGetLastError();
-      if (h == 0) { msg = cuda_msg("batch buffer allocation failed", e); return RM_ERR_ALLOC; }
-      parts = h;
-      enough = 0;
+      enough = false;
+      if (h > 0) {
+        parts = h;
+      } else {
+        if (!smaller_paths(c, room)) { msg = cuda_msg("batch buffer allocation failed", e); return RM_ERR_ALLOC; }
+        for (int k = 1; k < parts; ++k) ws[k]->release();  // what earlier batches left there
+      }
     }
   }
   cudaError_t e = cudaSuccess;

@@ -1,0 +1,81 @@
+"""Calls on a device whose memory is almost taken.
+
+What a call keeps only for speed it does without there, and its outputs stay the
+same: the plain frame and the batch take smaller chunks of samples or the lane
+kernels (rm_paths.cu, rm_kernels.cu).
+
+A child process makes its scenes, runs every call once at a small size, takes
+the device's memory but for a few megabytes with one tensor, runs the calls,
+gives the tensor back and runs them again."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CHILD = '''
+import sys
+import numpy as np, torch
+import raymotion_b200 as rb
+from raymotion_b200 import BatchItem, RenderConfig, _abi
+from raymotion_b200.scenes import PLAIN_FLAGS, sized_field
+
+WHAT, LEAVE = sys.argv[1], int(sys.argv[2]) << 20
+W, H = 1280, 720
+b = rb.Backend(0)
+sb, cam, _ = sized_field(5, 3000, 64, 36, 1, 4)
+scene = b.scene_create(sb.pack())
+
+
+def cfg(spp, w=W, h=H, adapt=0):
+    c = RenderConfig(width=w, height=h, spp=spp, max_bounces=3, restir_candidates=1, restir_spatial=0, flags=PLAIN_FLAGS)
+    c.adapt_min, c.adapt_step = adapt, 8 if spp < 32 else 32
+    return c
+
+
+hdr = [torch.empty(W * H * 3, device="cuda") for _ in range(3)]
+
+
+def frame(c, k=0):
+    hdr[k].zero_()
+    torch.cuda.synchronize()
+    b.render_scene_async(scene, cam, c, 7, None, hdr[k].data_ptr())
+    b.sync()
+    return hdr[k].cpu().numpy().copy()
+
+
+def batch(c):
+    b.render_batch([BatchItem(scene, cam, c, 30 + k, None, hdr[k].data_ptr(), None) for k in range(3)])
+    b.sync()
+    return np.stack([x.cpu().numpy() for x in hdr])
+
+
+frame(cfg(1))  # the frame's own buffers at their size
+for c in (cfg(8, 32, 18, 8), cfg(24, 32, 18, 8), cfg(64, 32, 18, 32), cfg(64, 32, 18), cfg(24, 320, 180, 8), cfg(64, 320, 180, 32)):
+    frame(c)  # every kernel once
+batch(cfg(16, 32, 18))
+calls = {"frame": lambda: [frame(cfg(4)), frame(cfg(16)), frame(cfg(16, adapt=8)), frame(cfg(64))],
+         "batch": lambda: [batch(cfg(16)), batch(cfg(3))]}[WHAT]
+taken = torch.empty(torch.cuda.mem_get_info()[0] - LEAVE, dtype=torch.uint8, device="cuda")
+left = torch.cuda.mem_get_info()[0]
+low = calls()
+del taken
+torch.cuda.empty_cache()
+full = calls()
+same = all(np.array_equal(a.view(np.uint32), c.view(np.uint32)) for a, c in zip(low, full))
+assert all(x.any() for x in full)
+print("LOW", left >> 20, "MB,", "same" if same else "different")
+'''
+
+
+@pytest.mark.parametrize("leave", [160, 48, 4])  # MB
+@pytest.mark.parametrize("what", ["frame", "batch"])
+def test_outputs_do_not_depend_on_free_memory(what, leave):
+    root = Path(__file__).resolve().parents[1]
+    r = subprocess.run([sys.executable, "-c", CHILD, what, str(leave)], capture_output=True, text=True, cwd=root,
+                       env=dict(os.environ, PYTHONPATH=str(root)), timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
+    assert "MB, same" in r.stdout, r.stdout
