@@ -890,7 +890,7 @@ size_t restir_generate_scratch(const Params& p, int sms) {
 cudaError_t launch_restir_generate(const Scene& s, const Params& p, uint64_t seed, const GBufSoA& gb, const ResSoA& ri,
                                    void* scratch, int sms, unsigned long long* ctr, uint32_t* err, cudaStream_t st) {
   const uint64_t npix = uint64_t(p.width) * uint64_t(p.height);
-  if (!gen_tiles(p, sms)) {
+  if (!scratch) {
     k_restir_generate<<<blocks_for(npix, 128), 128, 0, st>>>(s, p, seed, gb, ri, ctr, err);
     return cudaGetLastError();
   }

@@ -38,7 +38,8 @@ cudaError_t launch_paths(const Scene& s, const Params& p, uint64_t seed, const P
 // mode 0: every open pixel goes on, 1: those that fail the adaptive test, 2: none
 cudaError_t launch_paths_combine(const Params& p, const PathsArgs& a, int seg, int mode, int sms,
                                  cudaStream_t st);
-// K3; `scratch` holds restir_generate_scratch bytes
+// K3, in tiles with restir_generate_scratch bytes (0: not for this frame) of
+// scratch, a thread a pixel without (null)
 size_t restir_generate_scratch(const Params& p, int sms);
 cudaError_t launch_restir_generate(const Scene& s, const Params& p, uint64_t seed, const GBufSoA& gb, const ResSoA& ri,
                                    void* scratch, int sms, unsigned long long* ctr, uint32_t* err, cudaStream_t st);

@@ -755,7 +755,6 @@ int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_co
   const size_t npix = size_t(cfg.width) * size_t(cfg.height);
   cudaStream_t st = c->stream;
   cudaError_t e = ensure_frame(c, npix, pl.use_spatial);
-  if (e == cudaSuccess && pl.use_spatial) e = c->gen.reserve(restir_generate_scratch(p, c->sms));
   if (e != cudaSuccess) {
     msg = cuda_msg(pl.use_spatial ? "Metal ReSTIR buffer allocation failed" : "Metal image buffer allocation failed", e);
     return RM_ERR_ALLOC;
@@ -801,6 +800,11 @@ int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_co
     p.hasHistory = have_hist ? 1 : 0;
     p.prevCamera = c->hist_cam;
     const bool wavefront = !use_megakernel();  // ReSTIR scenes are opaque (make_plan)
+    void* gen = nullptr;
+    if (const size_t bytes = restir_generate_scratch(p, c->sms)) {
+      if (c->gen.reserve(bytes) == cudaSuccess) gen = c->gen.ptr;
+      else cudaGetLastError();  // no memory for tiles: a thread a pixel
+    }
     for (int stage = 0; stage < 3 && e == cudaSuccess; ++stage) {
       if (stage == 2 && wavefront) {
         std::string wmsg;
@@ -817,7 +821,7 @@ int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_co
       }
       e = staged(c, RM_STAGE_GENERATE + stage, [&] {
         if (stage == 0)
-          return launch_restir_generate(s, p, seed, c->gb.view(), c->rinit.view(), c->gen.ptr, c->sms,
+          return launch_restir_generate(s, p, seed, c->gb.view(), c->rinit.view(), gen, c->sms,
                                         ctr + 4 * RM_STAGE_GENERATE, err, st);
         return launch_restir_stage(stage, s, p, seed, c->gb.view(), c->rinit.view(), c->rmerged.view(), c->hg.view(),
                                    c->hres.view(), c->hdr.as<float>(), c->dbg.as<uint32_t>(),

@@ -2,7 +2,8 @@
 
 What a call keeps only for speed it does without there, and its outputs stay the
 same: the plain frame and the batch take smaller chunks of samples or the lane
-kernels (rm_paths.cu, rm_kernels.cu).
+kernels (rm_paths.cu, rm_kernels.cu), a small ReSTIR frame draws its candidates a
+thread a pixel instead of in tiles (rm_kernels.cu).
 
 A child process makes its scenes, runs every call once at a small size, takes
 the device's memory but for a few megabytes with one tensor, runs the calls,
@@ -53,12 +54,21 @@ def batch(c):
     return np.stack([x.cpu().numpy() for x in hdr])
 
 
+def restir(w, h):
+    c = RenderConfig(width=w, height=h, spp=1, max_bounces=3, restir_candidates=8, restir_spatial=2, adapt_min=0,
+                     flags=_abi.RM_FLAG_NO_ENV)
+    b.reset_history()
+    return frame(c)
+
+
+if WHAT == "restir":
+    restir(W, H)
 frame(cfg(1))  # the frame's own buffers at their size
 for c in (cfg(8, 32, 18, 8), cfg(24, 32, 18, 8), cfg(64, 32, 18, 32), cfg(64, 32, 18), cfg(24, 320, 180, 8), cfg(64, 320, 180, 32)):
     frame(c)  # every kernel once
 batch(cfg(16, 32, 18))
 calls = {"frame": lambda: [frame(cfg(4)), frame(cfg(16)), frame(cfg(16, adapt=8)), frame(cfg(64))],
-         "batch": lambda: [batch(cfg(16)), batch(cfg(3))]}[WHAT]
+         "batch": lambda: [batch(cfg(16)), batch(cfg(3))], "restir": lambda: [restir(333, 187)]}[WHAT]
 taken = torch.empty(torch.cuda.mem_get_info()[0] - LEAVE, dtype=torch.uint8, device="cuda")
 left = torch.cuda.mem_get_info()[0]
 low = calls()
@@ -72,7 +82,7 @@ print("LOW", left >> 20, "MB,", "same" if same else "different")
 
 
 @pytest.mark.parametrize("leave", [160, 48, 4])  # MB
-@pytest.mark.parametrize("what", ["frame", "batch"])
+@pytest.mark.parametrize("what", ["frame", "batch", "restir"])
 def test_outputs_do_not_depend_on_free_memory(what, leave):
     root = Path(__file__).resolve().parents[1]
     r = subprocess.run([sys.executable, "-c", CHILD, what, str(leave)], capture_output=True, text=True, cwd=root,
