@@ -161,6 +161,24 @@ Scene scene_view(const DevScene& sc) {
   return s;
 }
 
+// The staging copy of a scene's triangles that an upload of another kind leaves
+// allocated (giving it back waits for the device, which costs a small scene more
+// than its copy).
+constexpr size_t kStageKeep = size_t(32) << 20;
+constexpr const char* kTextureOutside = "triangle texture outside the texel array";
+
+// The host's form of check_triangles' texture test.
+static bool textures_inside(const rm_scene_view* sv) {
+  for (int i = 0; i < sv->n_tris; ++i) {
+    const rm_triangle& t = sv->tris[i];
+    if (t.texture_offset >= 0 &&
+        (t.texture_width <= 0 || t.texture_height <= 0 ||
+         int64_t(t.texture_offset) + int64_t(t.texture_width) * t.texture_height > sv->n_texels))
+      return false;
+  }
+  return true;
+}
+
 // Validate and upload one scene; build or convert its BVH.
 int upload_scene(rmcuda_ctx* c, DevScene& sc, const rm_scene_view* sv, std::string& msg) {
   NvtxRange range("rm scene upload");
@@ -185,22 +203,30 @@ int upload_scene(rmcuda_ctx* c, DevScene& sc, const rm_scene_view* sv, std::stri
     key += v ? v : "-";
     key += '|';
   }
-  const bool may_reuse = sc.have_scene && sc.device_built && !sv->nodes && sv->n_tris > 0 &&
-                         sv->n_tris == sc.n_tris && sc.bvh.n_records > 0 && key == sc.build_key;
   // The triangles go to the staging buffer when a resident scene must survive
   // their being rejected, else straight to their place, and their texture
   // ranges and opacity are checked on the device (the pass over them on the
-  // host took 2.4 ms for 400,000).
-  const bool stage = sc.have_scene && tb > 0;
+  // host took 2.4 ms for 400,000).  Without memory for a second copy that pass
+  // comes first and the triangles go straight to their place too.
+  bool stage = sc.have_scene && tb > 0;
+  if (stage && sc.tris_in.reserve(tb) != cudaSuccess) {
+    cudaGetLastError();
+    stage = false;
+    if (!textures_inside(sv)) { msg = kTextureOutside; return RM_ERR_INVALID; }
+  }
+  const bool may_reuse = stage && sc.device_built && !sv->nodes && sv->n_tris == sc.n_tris && sc.bvh.n_records > 0 &&
+                         key == sc.build_key;
   DevBuf& in = stage ? sc.tris_in : sc.tris;
   bool reuse = false, opaque = true;
   int word[2] = {0, 0};  // differ, check
   if ((e = in.reserve(tb)) != cudaSuccess || (e = c->hash_out.reserve(sizeof(word))) != cudaSuccess) {
+    if (!stage) sc.have_scene = false;
     msg = cuda_msg("Metal scene buffer allocation failed", e);
     return RM_ERR_ALLOC;
   }
   if (tb) {
     int* d_word = c->hash_out.as<int>();
+    if (!stage) sc.have_scene = false;
     if ((e = cudaMemcpyAsync(in.ptr, sv->tris, tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
         (may_reuse && (e = device_differ(in.ptr, sc.tris.ptr, tb, d_word, st)) != cudaSuccess) ||
         (e = check_triangles(in.as<rm_triangle>(), sv->n_tris, sv->n_texels, d_word + 1, st)) != cudaSuccess ||
@@ -211,16 +237,21 @@ int upload_scene(rmcuda_ctx* c, DevScene& sc, const rm_scene_view* sv, std::stri
     }
     reuse = may_reuse && word[0] == 0;
     if (word[1] & 2) {
-      msg = "triangle texture outside the texel array";  // the resident scene is untouched
+      msg = kTextureOutside;  // a resident scene is untouched
       return RM_ERR_INVALID;
     }
     opaque = !(word[1] & 1);
-    if (stage && !reuse) std::swap(sc.tris, sc.tris_in);
+    if (stage && !reuse) {
+      std::swap(sc.tris, sc.tris_in);
+      sc.have_scene = false;  // until its BVH is built
+      // a large old copy is kept only where the next upload may compare with it
+      if (!may_reuse && sc.tris_in.cap > kStageKeep) sc.tris_in.release();
+    }
   }
   if ((e = sc.lights.reserve(size_t(sv->n_lights) * 4)) != cudaSuccess ||
       (e = sc.cdf.reserve(size_t(sv->n_lights) * 4)) != cudaSuccess ||
       (e = sc.texels.reserve(size_t(sv->n_texels) * sizeof(rm_vec3))) != cudaSuccess) {
-    sc.have_scene = false;  // its triangles may be the new ones already
+    sc.have_scene = false;
     msg = cuda_msg("Metal scene buffer allocation failed", e);
     return RM_ERR_ALLOC;
   }

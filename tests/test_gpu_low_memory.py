@@ -3,7 +3,9 @@
 What a call keeps only for speed it does without there, and its outputs stay the
 same: the plain frame and the batch take smaller chunks of samples or the lane
 kernels (rm_paths.cu, rm_kernels.cu), a small ReSTIR frame draws its candidates a
-thread a pixel instead of in tiles (rm_kernels.cu).
+thread a pixel instead of in tiles (rm_kernels.cu), and a new upload of a scene
+checks the triangles before they take the place of the old ones, instead of beside
+them.
 
 A child process makes its scenes, runs every call once at a small size, takes
 the device's memory but for a few megabytes with one tensor, runs the calls,
@@ -61,6 +63,41 @@ def restir(w, h):
     return frame(c)
 
 
+def soup(n, seed):
+    from raymotion_b200.scene import SceneBuilder
+    r = np.random.default_rng(seed)
+    c = r.uniform(-20, 20, (n, 3)).astype(np.float32)
+    s = SceneBuilder()
+    s.add_triangles(c, c + r.normal(0, 0.3, (n, 3)), c + r.normal(0, 0.3, (n, 3)))
+    return s.pack()
+
+
+if WHAT == "upload":  # 70 MB of triangles; fewer; as many; one with a texture that is not there
+    scenes = [soup(400000, 1), soup(399000, 2), soup(399000, 3), soup(399000, 4)]
+    scenes[3].tris["texture_offset"][398999] = 0
+    r = np.random.default_rng(5)
+    rays = np.concatenate([r.uniform(-20, 20, (4096, 3)), r.normal(size=(4096, 3)), np.full((4096, 1), 50)], 1)
+    rays = torch.from_numpy(rays.astype(np.float32)).cuda()
+    tri = torch.empty(4096, dtype=torch.int32, device="cuda")
+
+    def hits():
+        b.trace(rays.data_ptr(), 4096, False, tri.data_ptr())
+        return tri.cpu().numpy() + 1  # (0: a miss)
+
+    def uploads():
+        out = []
+        for s in scenes[:3]:
+            b.upload(s, use_nodes=False)
+            out.append(hits())
+        try:
+            b.upload(scenes[3], use_nodes=False)
+            raise SystemExit("accepted")
+        except rb.RenderError as e:
+            assert "texture" in str(e), e
+        return out + [hits()]
+
+    b.upload(scenes[0], use_nodes=False)
+    hits()
 if WHAT == "restir":
     restir(W, H)
 frame(cfg(1))  # the frame's own buffers at their size
@@ -68,7 +105,8 @@ for c in (cfg(8, 32, 18, 8), cfg(24, 32, 18, 8), cfg(64, 32, 18, 32), cfg(64, 32
     frame(c)  # every kernel once
 batch(cfg(16, 32, 18))
 calls = {"frame": lambda: [frame(cfg(4)), frame(cfg(16)), frame(cfg(16, adapt=8)), frame(cfg(64))],
-         "batch": lambda: [batch(cfg(16)), batch(cfg(3))], "restir": lambda: [restir(333, 187)]}[WHAT]
+         "batch": lambda: [batch(cfg(16)), batch(cfg(3))], "restir": lambda: [restir(333, 187)],
+         "upload": lambda: uploads()}[WHAT]
 taken = torch.empty(torch.cuda.mem_get_info()[0] - LEAVE, dtype=torch.uint8, device="cuda")
 left = torch.cuda.mem_get_info()[0]
 low = calls()
@@ -82,7 +120,7 @@ print("LOW", left >> 20, "MB,", "same" if same else "different")
 
 
 @pytest.mark.parametrize("leave", [160, 48, 4])  # MB
-@pytest.mark.parametrize("what", ["frame", "batch", "restir"])
+@pytest.mark.parametrize("what", ["frame", "batch", "restir", "upload"])
 def test_outputs_do_not_depend_on_free_memory(what, leave):
     root = Path(__file__).resolve().parents[1]
     r = subprocess.run([sys.executable, "-c", CHILD, what, str(leave)], capture_output=True, text=True, cwd=root,
