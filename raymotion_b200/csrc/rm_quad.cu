@@ -65,13 +65,11 @@ __global__ void k_quad_init(int* roots, int* level_n, int levels) {
   if (i == 0) roots[0] = 0;
 }
 
-__global__ void __launch_bounds__(128) k_quad_level(const float4* __restrict__ rec, int level, int* roots,
-                                                    int* level_n, float4* __restrict__ quads) {
-  int begin = 0;
-  for (int l = 0; l < level; ++l) begin += level_n[l];
-  const int n_here = level_n[level];
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n_here; k += gridDim.x * blockDim.x) {
-    const int node = begin + k, r = roots[node];
+// The nodes [begin, begin + n_here) of a level; theirs to come follow them, counted in *next_n.
+__device__ __forceinline__ void collapse_level(const float4* __restrict__ rec, int begin, int n_here, int first,
+                                               int stride, int* roots, int* next_n, float4* __restrict__ quads) {
+  for (int k = first; k < n_here; k += stride) {
+    const int node = begin + k, r = __ldcg(roots + node);
     QChild ch[4];
     int n = 0;
     for (int s = 0; s < 2; ++s) {
@@ -104,7 +102,7 @@ __global__ void __launch_bounds__(128) k_quad_level(const float4* __restrict__ r
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (j < n && ch[j].cnt == 0) ++n_int;
-    int next = begin + n_here + (n_int ? atomicAdd(level_n + level + 1, n_int) : 0);
+    int next = begin + n_here + (n_int ? atomicAdd(next_n, n_int) : 0);
     uint32_t word[4];
     int src[4];
     float b[6][4];
@@ -133,6 +131,47 @@ __global__ void __launch_bounds__(128) k_quad_level(const float4* __restrict__ r
     reinterpret_cast<uint4*>(q)[6] = make_uint4(word[0], word[1], word[2], word[3]);
     reinterpret_cast<int4*>(q)[7] = make_int4(src[0], src[1], src[2], src[3]);
   }
+}
+
+__global__ void __launch_bounds__(128) k_quad_level(const float4* __restrict__ rec, int level, int* roots,
+                                                    int* level_n, float4* __restrict__ quads) {
+  int begin = 0;
+  for (int l = 0; l < level; ++l) begin += level_n[l];
+  collapse_level(rec, begin, level_n[level], int(blockIdx.x * blockDim.x + threadIdx.x), int(gridDim.x * blockDim.x),
+                 roots, level_n + level + 1, quads);
+}
+
+// The levels from `level` to the last, one block: a launch per level takes 4 us,
+// of which a small tree's levels use little and its empty ones (the binary
+// tree's depth is the bound) nothing.
+constexpr int kQuadRestThreads = 512;
+
+__global__ void __launch_bounds__(kQuadRestThreads) k_quad_rest(const float4* __restrict__ rec, int level, int levels,
+                                                                int* roots, int* level_n,
+                                                                float4* __restrict__ quads) {
+  __shared__ int next_n;
+  const int tid = int(threadIdx.x);
+  int begin = 0, n = 1;
+  if (level == 0 && tid == 0) roots[0] = 0;
+  if (level > 0) {
+    for (int l = 0; l < level; ++l) begin += level_n[l];
+    n = level_n[level];
+  }
+  int l = level;
+  for (; l < levels && n > 0; ++l) {
+    __syncthreads();
+    if (tid == 0) {
+      level_n[l] = n;
+      next_n = 0;
+    }
+    __syncthreads();
+    collapse_level(rec, begin, n, tid, kQuadRestThreads, roots, &next_n, quads);
+    __syncthreads();
+    begin += n;
+    n = next_n;
+  }
+  if (tid == 0)
+    for (; l < levels; ++l) level_n[l] = 0;
 }
 
 // One node per record, of its two children: node and record share their index.
@@ -194,14 +233,22 @@ cudaError_t build_quads(DevBvh& b, cudaStream_t st) {
                                                   b.quads.as<float4>());
     return cudaGetLastError();
   }
-  const int levels = std::max(1, std::min(b.max_depth, kStack));
-  k_quad_init<<<1, 128, 0, st>>>(roots, level_n, kStack + 2);
+  // One block takes a small tree whole and the levels behind the twelfth of a
+  // middling one (a caller's BVH of 60 and of 1,000 triangles uploaded: 90 and
+  // 120 us against 105 and 155 with a launch per level; 20,000: within the
+  // spread; a larger tree's late levels hold more than one block is fast with).
+  const int depth = std::max(1, std::min(b.max_depth, kStack));
+  const int launched = b.n_records <= 2048 ? 0 : b.n_records <= 65536 ? std::min(depth, 12) : depth;
+  if (launched > 0) k_quad_init<<<1, 128, 0, st>>>(roots, level_n, kStack + 2);
   long long most = 1;
-  for (int l = 0; l < levels; ++l) {
+  for (int l = 0; l < launched; ++l) {
     const long long blocks = std::min<long long>(148 * 8, (std::min<long long>(most, bound) + 127) / 128);
     k_quad_level<<<unsigned(blocks), 128, 0, st>>>(b.records.as<float4>(), l, roots, level_n, b.quads.as<float4>());
     most = std::min<long long>(most * 4, bound);
   }
+  if (launched < depth)
+    k_quad_rest<<<1, kQuadRestThreads, 0, st>>>(b.records.as<float4>(), launched, kStack + 2, roots, level_n,
+                                                b.quads.as<float4>());
   return cudaGetLastError();
 }
 
