@@ -165,18 +165,21 @@ Scene scene_view(const DevScene& sc) {
 // allocated (giving it back waits for the device, which costs a small scene more
 // than its copy).
 constexpr size_t kStageKeep = size_t(32) << 20;
+constexpr int kHostCheck = 2048;  // triangles: 12 us on the host
 constexpr const char* kTextureOutside = "triangle texture outside the texel array";
 
-// The host's form of check_triangles' texture test.
-static bool textures_inside(const rm_scene_view* sv) {
+// The host's form of check_triangles.
+static int check_triangles_host(const rm_scene_view* sv) {
+  int f = 0;
   for (int i = 0; i < sv->n_tris; ++i) {
     const rm_triangle& t = sv->tris[i];
+    if (!(t.alpha >= 1.0f)) f |= 1;
     if (t.texture_offset >= 0 &&
         (t.texture_width <= 0 || t.texture_height <= 0 ||
          int64_t(t.texture_offset) + int64_t(t.texture_width) * t.texture_height > sv->n_texels))
-      return false;
+      f |= 2;
   }
-  return true;
+  return f;
 }
 
 // Validate and upload one scene; build or convert its BVH.
@@ -203,35 +206,43 @@ int upload_scene(rmcuda_ctx* c, DevScene& sc, const rm_scene_view* sv, std::stri
     key += v ? v : "-";
     key += '|';
   }
-  // The triangles go to the staging buffer when a resident scene must survive
-  // their being rejected, else straight to their place, and their texture
-  // ranges and opacity are checked on the device (the pass over them on the
-  // host took 2.4 ms for 400,000).  Without memory for a second copy that pass
-  // comes first and the triangles go straight to their place too.
-  bool stage = sc.have_scene && tb > 0;
+  bool may_reuse = sc.have_scene && sc.device_built && !sv->nodes && sv->n_tris > 0 && sv->n_tris == sc.n_tris &&
+                   sc.bvh.n_records > 0 && key == sc.build_key;
+  // Texture ranges and opacity are checked on the host for a small scene, else
+  // on the device (400,000 triangles took 2.4 ms on the host; the check's launches
+  // and the wait take 20 us).  The triangles go to the staging buffer when they
+  // may equal the resident ones, or when a resident scene must survive their
+  // being rejected by the device, and straight to their place otherwise.
+  // Without memory for the second copy the host checks them all.
+  bool on_host = sv->n_tris <= kHostCheck;
+  bool stage = may_reuse || (sc.have_scene && tb > 0 && !on_host);
   if (stage && sc.tris_in.reserve(tb) != cudaSuccess) {
     cudaGetLastError();
-    stage = false;
-    if (!textures_inside(sv)) { msg = kTextureOutside; return RM_ERR_INVALID; }
+    stage = may_reuse = false;
+    on_host = true;
   }
-  const bool may_reuse = stage && sc.device_built && !sv->nodes && sv->n_tris == sc.n_tris && sc.bvh.n_records > 0 &&
-                         key == sc.build_key;
+  int word[2] = {0, on_host ? check_triangles_host(sv) : 0};  // differ, check
   DevBuf& in = stage ? sc.tris_in : sc.tris;
-  bool reuse = false, opaque = true;
-  int word[2] = {0, 0};  // differ, check
+  bool reuse = false;
+  if (word[1] & 2) {
+    msg = kTextureOutside;  // a resident scene is untouched
+    return RM_ERR_INVALID;
+  }
+  if (!stage) sc.have_scene = false;
   if ((e = in.reserve(tb)) != cudaSuccess || (e = c->hash_out.reserve(sizeof(word))) != cudaSuccess) {
-    if (!stage) sc.have_scene = false;
     msg = cuda_msg("Metal scene buffer allocation failed", e);
     return RM_ERR_ALLOC;
   }
   if (tb) {
     int* d_word = c->hash_out.as<int>();
-    if (!stage) sc.have_scene = false;
+    const int first = may_reuse ? 0 : 1, last = on_host ? 0 : 1;  // the words that the device answers
     if ((e = cudaMemcpyAsync(in.ptr, sv->tris, tb, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
         (may_reuse && (e = device_differ(in.ptr, sc.tris.ptr, tb, d_word, st)) != cudaSuccess) ||
-        (e = check_triangles(in.as<rm_triangle>(), sv->n_tris, sv->n_texels, d_word + 1, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(word, d_word, sizeof(word), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(st)) != cudaSuccess) {
+        (!on_host && (e = check_triangles(in.as<rm_triangle>(), sv->n_tris, sv->n_texels, d_word + 1, st)) !=
+                         cudaSuccess) ||
+        (first <= last && ((e = cudaMemcpyAsync(word + first, d_word + first, size_t(last - first + 1) * sizeof(int),
+                                                cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+                           (e = cudaStreamSynchronize(st)) != cudaSuccess))) {
       msg = cuda_msg("scene upload failed", e);
       return RM_ERR_CUDA;
     }
@@ -240,7 +251,6 @@ int upload_scene(rmcuda_ctx* c, DevScene& sc, const rm_scene_view* sv, std::stri
       msg = kTextureOutside;  // a resident scene is untouched
       return RM_ERR_INVALID;
     }
-    opaque = !(word[1] & 1);
     if (stage && !reuse) {
       std::swap(sc.tris, sc.tris_in);
       sc.have_scene = false;  // until its BVH is built
@@ -248,6 +258,7 @@ int upload_scene(rmcuda_ctx* c, DevScene& sc, const rm_scene_view* sv, std::stri
       if (!may_reuse && sc.tris_in.cap > kStageKeep) sc.tris_in.release();
     }
   }
+  const bool opaque = !(word[1] & 1);
   if ((e = sc.lights.reserve(size_t(sv->n_lights) * 4)) != cudaSuccess ||
       (e = sc.cdf.reserve(size_t(sv->n_lights) * 4)) != cudaSuccess ||
       (e = sc.texels.reserve(size_t(sv->n_texels) * sizeof(rm_vec3))) != cudaSuccess) {
