@@ -167,11 +167,7 @@ __global__ void k_pack_tgeo(const rm_triangle* __restrict__ tris, const int32_t*
                             float4* __restrict__ tgeo) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int j = order[i];
-  const rm_triangle& t = tris[j];
-  tgeo[size_t(i) * 3 + 0] = make_float4(t.v0.x, t.v0.y, t.v0.z, __int_as_float(j));
-  tgeo[size_t(i) * 3 + 1] = make_float4(t.v1.x - t.v0.x, t.v1.y - t.v0.y, t.v1.z - t.v0.z, 0.f);
-  tgeo[size_t(i) * 3 + 2] = make_float4(t.v2.x - t.v0.x, t.v2.y - t.v0.y, t.v2.z - t.v0.z, 0.f);
+  pack_record(tris[order[i]], order[i], tgeo + size_t(i) * 3);
 }
 
 // Refit: one thread per record; leaf slots are boxed from their triangles,
@@ -687,9 +683,7 @@ cudaError_t refit_bvh(const rm_triangle* d_tris, DevBvh& bvh, cudaStream_t st) {
                                                        bvh.parents.as<int32_t>(), bvh.counters.as<int>(),
                                                        bvh.n_records);
   e = cudaGetLastError();
-  if (e == cudaSuccess) e = refit_quads(bvh, st);
-  if (e != cudaSuccess) return e;
-  return pack_tgeo(d_tris, bvh, st);
+  return e == cudaSuccess ? refit_last(d_tris, bvh, st) : e;
 }
 
 cudaError_t check_triangles(const rm_triangle* d_tris, int n, long long n_texels, int* d_flags, cudaStream_t st) {

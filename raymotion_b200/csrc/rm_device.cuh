@@ -191,6 +191,13 @@ struct Bsdf { float r, g, b, pdf; };
 // the Moller-Trumbore test would accept: the hit is independent of the BVH.
 struct TraceResult { float t; int tri; float u, v; };
 
+// A triangle's record: first vertex and index, then its two edges.
+__device__ __forceinline__ void pack_record(const rm_triangle& t, int j, float4* g) {
+  g[0] = make_float4(t.v0.x, t.v0.y, t.v0.z, __int_as_float(j));
+  g[1] = make_float4(t.v1.x - t.v0.x, t.v1.y - t.v0.y, t.v1.z - t.v0.z, 0.f);
+  g[2] = make_float4(t.v2.x - t.v0.x, t.v2.y - t.v0.y, t.v2.z - t.v0.z, 0.f);
+}
+
 // Moller-Trumbore against one triangle record (pathtrace.metal:150-158) with
 // the (t, triangle index) order of the header; true when it became the hit.
 __device__ __forceinline__ bool test_triangle(const float4* __restrict__ g, float ox, float oy, float oz, float dx,

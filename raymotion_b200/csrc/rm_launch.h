@@ -285,9 +285,11 @@ cudaError_t pack_tgeo(const rm_triangle* d_tris, DevBvh& bvh, cudaStream_t st);
 // Refit all boxes bottom-up from the current triangle positions.
 cudaError_t refit_bvh(const rm_triangle* d_tris, DevBvh& bvh, cudaStream_t st);
 // Collapse the binary records (of a tree of depth max_depth) into the 4-wide
-// BVH, and copy their boxes into it after a refit (rm_quad.cu).
+// BVH (rm_quad.cu).
 cudaError_t build_quads(DevBvh& bvh, cudaStream_t st);
-cudaError_t refit_quads(DevBvh& bvh, cudaStream_t st);
+// After a refit of the records: their boxes into the 4-wide BVH and the
+// triangles into the leaf-ordered records.
+cudaError_t refit_last(const rm_triangle* d_tris, DevBvh& bvh, cudaStream_t st);
 // Collapse the binary records into the 8-wide compressed BVH (rm_wide.cu).
 // Leaves n_wide at 0 (the binary BVH stays in use) when a node cannot be
 // encoded, the wide tree would be deeper than the traversal stack, or the
