@@ -565,13 +565,21 @@ __device__ __noinline__ HeldLight held_light(const Params& p, const ResSoA& rm, 
 // bsdf_grad, the additions, no alpha code in opaque scenes): that frame's
 // adjoint 21.8 -> 18.9 ms by the loop, -> 17.1 by the copies.  Sixteen warps an
 // SM (12: +0.6 ms, 20: no change).  One block of 512 threads: 4 of 128 take the
-// same time but add 592 partial sums to each gradient instead of 148 (rounding
-// 2.9e-7 of the gradient instead of 2.0e-7, 256 x 256 x 16 spp).
+// same time but add 592 partial sums to each gradient instead of 148.
 constexpr int kAdjThreads = 512, kAdjBlocks = 1;
 constexpr int kAdjRefill = 16;  // idle lanes of a warp that make it take new pixel lanes
-// Pixel lanes that a warp takes between two passes of its block's sums to the
-// gradient, so that the 32-bit sums stay as short as those of a block that
-// owned 256 pixel lanes.
+
+// A block's sums are of 32 bits, and so is the gradient: a sum of many terms and
+// many sums are both inexact.  So a block holds two arrays of sums where they
+// fit in 32 KB: terms go to the first, which passes on to the second about each
+// time the block has taken this many pixel lanes (a warp's turn comes every 256
+// of its own, the warps' turns evenly spread), and the second goes to the gradient
+// at the end.  (One array passes on to the gradient itself.)
+// Error against the sum of 64 bands' gradients in 64 bits: 512x512, 32 spp 2.0e-7
+// of the gradient, 1024x1024, 32 spp 1.9e-7; with the first array passed on to the
+// gradient 1.1e-6 and 1.4e-6, with one that is never passed on 3.0e-7 and 4.5e-7,
+// but 1.6e-3 where all terms are equal (1024x1024, 100 spp), which the two
+// hold to 8e-6.  The second array costs 1 % (10.68 -> 10.77 ms at 512x512).
 constexpr unsigned kAdjFlush = 256;
 
 struct AdjointArgs {
@@ -580,22 +588,36 @@ struct AdjointArgs {
   const float* dLdI;
   const float* dLdalb;  // kRestir: through the denoiser's weights, or null
   float* grad;
-  int use_shared, lanes;
+  int sums, lanes;  // sums: arrays of n_mat x 8 sums in the block's memory (0: none)
+  unsigned flush;   // pixel lanes of a warp between its turns to pass the sums on
   unsigned* next;
   unsigned long long* ctr;
   uint32_t* err;
 };
 
+// By one warp; a copy of its own, called seldom.
+__device__ __noinline__ void pass_sums_on(const AdjointArgs& a) {
+  const int n = a.n_mat * kMatParams;
+#pragma unroll 1
+  for (int i = int(threadIdx.x & 31); i < n; i += 32) {
+    const float v = sh_sums[i] != 0.0f ? atomicExch(sh_sums + i, 0.0f) : 0.0f;
+    if (v == 0.0f) continue;
+    if (a.sums == 2) atomicAdd(sh_sums + n + i, v);
+    else atomicAdd(a.grad + i, v);
+  }
+}
+
 template <int kNee, bool kRestir>
 __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks) k_adjoint(Scene s, Params p, uint64_t seed, GBufSoA gb,
                                                                      ResSoA rm, AdjointArgs a) {
   float* sh = sh_sums;
-  if (a.use_shared) {
-    for (int i = threadIdx.x; i < a.n_mat * kMatParams; i += blockDim.x) sh[i] = 0.0f;
+  const int n_sums = a.n_mat * kMatParams;
+  if (a.sums > 0) {
+    for (int i = threadIdx.x; i < n_sums * a.sums; i += blockDim.x) sh[i] = 0.0f;
     __syncthreads();
   }
   const unsigned full = 0xffffffffu;
-  const GradSink sink{a.use_shared != 0, a.grad};
+  const GradSink sink{a.sums > 0, a.grad};
   const int lane_id = int(threadIdx.x & 31);
   const unsigned L = unsigned(a.lanes);
   const unsigned tasks = unsigned(p.width) * unsigned(p.height) * L;
@@ -605,7 +627,9 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks) k_adjoint(Scene s, Pa
   Walk w;
   Kept kept;
   bool active = false, fresh = false, again = false, more = true, indirect = false;
-  unsigned taken = 0;  // by the warp since it last passed the block's sums on
+  // pixel lanes that the warp took since it last passed the block's sums on; its
+  // turns lie evenly between the other warps'
+  unsigned taken = threadIdx.x / 32 * (a.flush / (blockDim.x / 32));
   // mode of the walk: 0 the only one (terms kept), 1 with C known, 2 for C alone
   int mode = 0, si = 0;
   uint32_t id = 0, start_state = 0, samples = 0;
@@ -622,12 +646,9 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks) k_adjoint(Scene s, Pa
       if (lane_id == 0) first = atomicAdd(a.next, unsigned(__popc(idle)));
       first = __shfl_sync(full, first, 0);
       taken += unsigned(__popc(idle));
-      if (a.use_shared && taken >= kAdjFlush) {
-        taken = 0;
-        for (int i = lane_id; i < a.n_mat * kMatParams; i += 32) {
-          const float v = sh[i] != 0.0f ? atomicExch(sh + i, 0.0f) : 0.0f;
-          if (v != 0.0f) atomicAdd(a.grad + i, v);
-        }
+      if (taken >= a.flush) {
+        taken -= a.flush;
+        pass_sums_on(a);
       }
       more = first + unsigned(__popc(idle)) < tasks;
       const unsigned t = first + unsigned(__popc(idle & ((1u << lane_id) - 1u)));
@@ -834,10 +855,12 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks) k_adjoint(Scene s, Pa
   __syncwarp();
   const unsigned long long tot = __reduce_add_sync(full, samples);
   if (lane_id == 0 && tot) atomicAdd(a.ctr, tot);
-  if (a.use_shared) {
+  if (a.sums > 0) {
     __syncthreads();
-    for (int i = threadIdx.x; i < a.n_mat * kMatParams; i += blockDim.x)
-      if (sh[i] != 0.0f) atomicAdd(a.grad + i, sh[i]);
+    for (int i = threadIdx.x; i < n_sums; i += blockDim.x) {
+      const float v = a.sums == 2 ? sh[n_sums + i] + sh[i] : sh[i];
+      if (v != 0.0f) atomicAdd(a.grad + i, v);
+    }
   }
 }
 
@@ -863,16 +886,24 @@ namespace {
 template <bool kRestir>
 cudaError_t run_adjoint(const Scene& s, const Params& p, uint64_t seed, const GBufSoA& gb, const ResSoA& rm,
                         AdjointArgs a, int sms, cudaStream_t st) {
-  const size_t shmem = size_t(a.n_mat) * kMatParams * sizeof(float);
-  a.use_shared = shmem <= 32 * 1024 ? 1 : 0;
+  const size_t one = size_t(a.n_mat) * kMatParams * sizeof(float);
+  a.sums = one * 2 <= 32 * 1024 ? 2 : one <= 32 * 1024 ? 1 : 0;
   const size_t threads = size_t(p.width) * size_t(p.height) * size_t(a.lanes);
+  a.flush = kAdjFlush;
   // fewer pixel lanes than the GPU's threads: narrower blocks, one on each SM
   // (64x64, 2 spp 0.72 ms against 0.84, its ReSTIR frame 1.30 / 1.51, 130x97, 8
   // spp 4.04 / 4.50)
   const size_t per_sm = (threads + size_t(sms) * 32 - 1) / (size_t(sms) * 32) * 32;
   const unsigned block = unsigned(std::min<size_t>(kAdjThreads, per_sm));
   const unsigned grid = unsigned(std::min<size_t>(size_t(sms) * kAdjBlocks, (threads + block - 1) / block));
-  const size_t sm = a.use_shared ? shmem : 0;
+  if (threads <= size_t(grid) * kAdjFlush && a.sums == 2) {
+    // a block takes no more than one pass: the first array does (64x64 on the
+    // ReSTIR chain 3.2 ms, with the second's memory gone from the cache 3.7)
+    a.sums = 1;
+    a.flush = 0xffffffffu;
+  }
+  if (a.sums == 0) a.flush = 0xffffffffu;
+  const size_t sm = size_t(a.sums) * one;
   const cudaError_t e = cudaMemsetAsync(a.next, 0, sizeof(unsigned), st);
   if (e != cudaSuccess) return e;
   if (!kRestir && !p.opaque) k_adjoint<1, false><<<grid, block, sm, st>>>(s, p, seed, gb, rm, a);
@@ -887,7 +918,7 @@ cudaError_t launch_adjoint(int lanes, const Scene& s, const Params& p, uint64_t 
                            int n_mat, const float* dLdI, float* grad, unsigned* next, int sms, unsigned long long* ctr,
                            uint32_t* err, cudaStream_t st) {
   return run_adjoint<false>(s, p, seed, GBufSoA{}, ResSoA{},
-                            AdjointArgs{tri_mat, n_mat, dLdI, nullptr, grad, 0, lanes, next, ctr, err}, sms, st);
+                            AdjointArgs{tri_mat, n_mat, dLdI, nullptr, grad, 0, lanes, 0, next, ctr, err}, sms, st);
 }
 
 cudaError_t apply_materials(rm_triangle* tris, const int32_t* tri_mat, const float* mats, int n_tris,
@@ -902,7 +933,7 @@ cudaError_t launch_adjoint_restir(const Scene& s, const Params& p, uint64_t seed
                                   float* grad, unsigned* next, int sms, unsigned long long* ctr, uint32_t* err,
                                   cudaStream_t st) {
   return run_adjoint<true>(s, p, seed, gb, rm,
-                           AdjointArgs{tri_mat, n_mat, dLdI, dLdalb, grad, 0, 1, next, ctr, err}, sms, st);
+                           AdjointArgs{tri_mat, n_mat, dLdI, dLdalb, grad, 0, 1, 0, next, ctr, err}, sms, st);
 }
 
 }  // namespace rmd
