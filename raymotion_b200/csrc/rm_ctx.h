@@ -135,6 +135,9 @@ struct rmcuda_ctx {
   rmd::DevBuf hdr, tmp_a, tmp_b, hist_col, rgb, dbg, hash_out;
   rmd::DevBuf ctr, err;
   rmd::DevBuf paths;  // values, states, sums and lists of a plain frame (rm_paths.cu)
+  // pinned, a word per stream: the last chunk of a plain frame found without an open pixel
+  unsigned long long* h_done = nullptr;
+  unsigned long long ticket = 0;  // chunks so far
   int sms = 0;
   // speculative frames of rmcuda_render: the copy stream that uploads and
   // compares the triangles while the frame renders, its pinned result, a copy
@@ -280,6 +283,7 @@ struct PathsTarget {
   float* hdr;
   uint8_t* rgb;
   uint32_t* dbg;
+  int part;    // of the context's streams
   int stage;   // whose counters the image's work adds to
   bool timed;  // by the profiler, on the context stream
 };

@@ -35,9 +35,10 @@ struct PathsArgs {
 long long paths_one_wave(int sms);  // lanes of one wave of resident blocks
 cudaError_t launch_paths(const Scene& s, const Params& p, uint64_t seed, const PathsArgs& a, int seg, int sms,
                          unsigned long long* ctr, uint32_t* err, cudaStream_t st);
-// mode 0: every open pixel goes on, 1: those that fail the adaptive test, 2: none
-cudaError_t launch_paths_combine(const Params& p, const PathsArgs& a, int seg, int mode, int sms,
-                                 cudaStream_t st);
+// mode 0: every open pixel goes on, 1: those that fail the adaptive test, 2: none.
+// done: host memory (or null) that gets `ticket` when the segment has no open pixel
+cudaError_t launch_paths_combine(const Params& p, const PathsArgs& a, int seg, int mode, unsigned long long* done,
+                                 unsigned long long ticket, int sms, cudaStream_t st);
 // K3, in tiles with restir_generate_scratch bytes (0: not for this frame) of
 // scratch, a thread a pixel without (null)
 size_t restir_generate_scratch(const Params& p, int sms);

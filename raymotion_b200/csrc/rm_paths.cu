@@ -192,8 +192,13 @@ __global__ void __launch_bounds__(kPathThreads, kPathBlocks) k_paths(Scene s, Pa
 // adaptive test (:806-810) and either the pixel's output (:811-814) or its
 // entry in the next segment's list.
 template <int L>
-__global__ void __launch_bounds__(256) k_paths_combine(Params p, PathsArgs a, int seg, int mode) {
+__global__ void __launch_bounds__(256) k_paths_combine(Params p, PathsArgs a, int seg, int mode,
+                                                       unsigned long long* done, unsigned long long ticket) {
   const int n_open = seg == 0 ? a.n_pixels : a.counts[seg];
+  if (n_open == 0) {
+    if (done && blockIdx.x == 0 && threadIdx.x == 0) *static_cast<volatile unsigned long long*>(done) = ticket;
+    return;
+  }
   const int* list = seg == 0 ? nullptr : a.list[seg & 1];
   const int lane = int(threadIdx.x & 31) % L;
   const int stride = int(gridDim.x * blockDim.x) / L;
@@ -272,12 +277,12 @@ cudaError_t launch_paths(const Scene& s, const Params& p, uint64_t seed, const P
   return run<2>(s, p, seed, a, seg, blocks, ctr, err, st);
 }
 
-cudaError_t launch_paths_combine(const Params& p, const PathsArgs& a, int seg, int mode, int sms,
-                                 cudaStream_t st) {
+cudaError_t launch_paths_combine(const Params& p, const PathsArgs& a, int seg, int mode, unsigned long long* done,
+                                 unsigned long long ticket, int sms, cudaStream_t st) {
   const long long threads = (long long)a.n_pixels * a.lanes;
   const unsigned g = unsigned(std::min<long long>((long long)sms * 8, (threads + 255) / 256));
-  if (a.lanes == 8) k_paths_combine<8><<<g, 256, 0, st>>>(p, a, seg, mode);
-  else k_paths_combine<32><<<g, 256, 0, st>>>(p, a, seg, mode);
+  if (a.lanes == 8) k_paths_combine<8><<<g, 256, 0, st>>>(p, a, seg, mode, done, ticket);
+  else k_paths_combine<32><<<g, 256, 0, st>>>(p, a, seg, mode, done, ticket);
   return cudaGetLastError();
 }
 

@@ -421,7 +421,7 @@ int run_own(rmcuda_ctx* c, const std::vector<BtJob>& jobs, std::string& msg) {
     const BtJob& J = jobs[i];
     const int h = part[i];
     e = run_paths(c, J.s, J.p, J.lanes, J.seed, plans[i],
-                  PathsTarget{*ws[h], sts[h], J.hdr, J.rgb, J.dbg, RM_STAGE_BATCH, false});
+                  PathsTarget{*ws[h], sts[h], J.hdr, J.rgb, J.dbg, h, RM_STAGE_BATCH, false});
   }
   for (int h = 1; h < parts; ++h) {
     if (e == cudaSuccess) e = cudaEventRecord(c->ev_join[h - 1], sts[h]);

@@ -131,3 +131,38 @@ def test_large_sample_counts_equal_the_oracle(backend, oracle, w, h, spp):
     assert np.array_equal(hdr.view(np.uint32), np.asarray(o_hdr).reshape(-1).view(np.uint32))
     assert np.array_equal(rgb, o_rgb)
     assert np.array_equal(backend.debug_read(4, w * h), o.debug_read(4, w * h))
+
+
+def test_frames_whose_pixels_stop_early(backend, oracle):
+    """Frames of many segments whose adaptive test soon stops every pixel, the
+    rest of whose launches the host may save, between frames that go on, alone and
+    in a batch on several streams: all equal the oracle."""
+    import torch
+
+    from . import kat_scenes as K
+    even = oracle.with_reference_bvh(K.fullscreen_emitter())
+    noisy = oracle.with_reference_bvh(cornell_box(3)[0].pack())
+    cam = cornell_box(3)[1]
+    cfgs = {id(even): _plain(160, 90, 512, 2, adapt=(16, 8)), id(noisy): _plain(40, 30, 96, 3, adapt=(16, 8))}
+    for c in cfgs.values():
+        c.adapt_rel, c.adapt_abs = 0.02, 0.002
+    order = [even, noisy, even, even, noisy, noisy, even, noisy]
+    want = {id(s): oracle.Oracle().render(s, cam, cfgs[id(s)], 5)[1].reshape(-1) for s in (even, noisy)}
+    handles = {id(s): backend.scene_create(s) for s in (even, noisy)}
+    try:
+        outs = [torch.empty(cfgs[id(s)].width * cfgs[id(s)].height * 3, device="cuda") for s in order]
+        for s, o in zip(order, outs):  # one after the other, not waited for
+            backend.render_scene_async(handles[id(s)], cam, cfgs[id(s)], 5, None, o.data_ptr())
+        backend.sync()
+        alone = [o.cpu().numpy() for o in outs]
+        for o in outs:
+            o.zero_()
+        backend.render_batch([BatchItem(handles[id(s)], cam, cfgs[id(s)], 5, None, o.data_ptr(), None)
+                              for s, o in zip(order, outs)])
+        for s, a, o in zip(order, alone, outs):
+            ref = np.asarray(want[id(s)], np.float32)
+            assert np.array_equal(a.view(np.uint32), ref.view(np.uint32))
+            assert np.array_equal(o.cpu().numpy().view(np.uint32), ref.view(np.uint32))
+    finally:
+        for h in handles.values():
+            backend.scene_destroy(h)
