@@ -731,6 +731,7 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
     k_single_leaf<<<1, 1, 0, st>>>(d_tris, n, b.records.as<float4>(), b.parents.as<int>(), b.order.as<int>());
     RM_TRY(cudaGetLastError());
     b.max_depth = 1;
+    b.shared = false;
     b.tree = true;
     b.leaf_tris = n;
     RM_TRY(build_quads(b, st));
@@ -785,6 +786,7 @@ cudaError_t build_lbvh(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   RM_TRY(cudaMemcpyAsync(&b.max_depth, b.depth.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
   RM_TRY(cudaStreamSynchronize(st));
   if (b.max_depth > kStack) { err = "device BVH deeper than the traversal stack"; return cudaErrorInvalidValue; }
+  b.shared = false;
   b.tree = true;
   b.leaf_tris = n;
   RM_TRY(build_quads(b, st));
@@ -1340,6 +1342,7 @@ cudaError_t build_ploc(const rm_triangle* d_tris, int n, int leaf_max, DevBvh& b
   b.max_depth = built[0];
   if (b.max_depth > kStack) { err = "device BVH deeper than the traversal stack"; return cudaErrorInvalidValue; }
   b.n_records = n - 1;
+  b.shared = false;
   b.tree = true;
   b.leaf_tris = n;
   RM_TRY(build_quads(b, st));
@@ -1443,6 +1446,7 @@ bool convert_caller_bvh(const rm_bvh_node* nodes, int M, const int32_t* bvh_tri,
     if (size[0] >= double(kMaxLink)) { err = "BVH exceeds 16777215 nodes with its shared subtrees written out"; return false; }
   }
   out.max_depth = max_depth;
+  out.shared = shared;
   out.tree = !shared && nested;
   out.leaf_tris = leaf_tris;
   out.n_records = n_rec;

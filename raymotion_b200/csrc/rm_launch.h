@@ -256,6 +256,7 @@ struct DevBvh {
   int n_records = 0;
   int n_tris = 0;
   int max_depth = 0;
+  bool shared = false;  // a node of a caller's BVH has several parents: no refit (parents holds one)
   // The records may be collapsed: every node has one parent, and its box is
   // ordered and inside its parent's (a caller's BVH may break either).
   bool tree = true;

@@ -1064,7 +1064,7 @@ int rmcuda_scene_update(rmcuda_ctx* c, const rm_triangle* tris, int32_t n, int32
   e = prepare_lights(c->sc.tris.as<rm_triangle>(), c->sc.lights.as<int32_t>(), c->sc.cdf.as<float>(), c->sc.n_lights,
                      c->sc.light_total, c->sc.lrec, c->sc.guide, c->sc.guide_n, c->sc.guide_inv, c->stream);
   if (e != cudaSuccess) { set_err(err, errcap, cuda_msg("light preparation failed", e)); return RM_ERR_CUDA; }
-  if (rebuild_every > 0 && c->sc.refits + 1 >= rebuild_every) {
+  if (c->sc.bvh.shared || (rebuild_every > 0 && c->sc.refits + 1 >= rebuild_every)) {
     std::string berr;
     e = build_device_bvh(c->sc.tris.as<rm_triangle>(), n, c->sc.bvh, c->stream, berr);
     c->sc.refits = 0;

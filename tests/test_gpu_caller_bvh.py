@@ -176,3 +176,19 @@ def test_boxes_are_taken_as_given(backend, oracle, what, wide, monkeypatch):
         assert 0 < hit.mean() < every
     else:
         assert _check(backend, oracle, caller, rays) == every
+
+
+@pytest.mark.parametrize("shape", list(SHARED))
+def test_update_of_shared_subtrees(backend, oracle, shape):
+    """A subtree with several parents has no one place to pass its new box on to."""
+    n, root = SHARED[shape]
+    sc = oracle.with_reference_bvh(_soup(n, 31, spread=1.0))
+    backend.upload(caller_bvh(sc, root()), use_nodes=True)
+    moved = sc.tris.copy()
+    for f in ("v0", "v1", "v2"):
+        moved[f] += np.float32(3.0)
+    backend.update(moved, rebuild_every=0)
+    v64 = np.concatenate([moved["v0"], moved["v1"], moved["v2"]], axis=1).astype(np.float64)
+    ms = oracle.with_reference_bvh(type(sc)(tris=moved, light_tri=sc.light_tri, light_cdf=sc.light_cdf,
+                                            light_total=sc.light_total, texels=sc.texels, verts64=v64))
+    assert _check(backend, oracle, ms, random_rays(4000, [1, 1, 1], [5, 5, 5], n)) > 0.0
