@@ -579,7 +579,8 @@ constexpr int kAdjRefill = 16;  // idle lanes of a warp that make it take new pi
 // of the gradient, 1024x1024, 32 spp 1.9e-7; with the first array passed on to the
 // gradient 1.1e-6 and 1.4e-6, with one that is never passed on 3.0e-7 and 4.5e-7,
 // but 1.6e-3 where all terms are equal (1024x1024, 100 spp), which the two
-// hold to 8e-6.  The second array costs 1 % (10.68 -> 10.77 ms at 512x512).
+// hold to 9e-6.  The second array costs nothing at 512x512, 32 spp (10.65 ms) and
+// 2 % at 256x256, 16 spp (2.40 -> 2.44).
 constexpr unsigned kAdjFlush = 256;
 
 struct AdjointArgs {
@@ -595,15 +596,15 @@ struct AdjointArgs {
   uint32_t* err;
 };
 
-// By one warp; a copy of its own, called seldom.
-__device__ __noinline__ void pass_sums_on(const AdjointArgs& a) {
-  const int n = a.n_mat * kMatParams;
+// The block's n sums to its second array (grad null) or to the gradient, by one
+// warp; a copy of its own, called seldom.
+__device__ __noinline__ void pass_sums_on(int n, float* grad) {
 #pragma unroll 1
   for (int i = int(threadIdx.x & 31); i < n; i += 32) {
     const float v = sh_sums[i] != 0.0f ? atomicExch(sh_sums + i, 0.0f) : 0.0f;
     if (v == 0.0f) continue;
-    if (a.sums == 2) atomicAdd(sh_sums + n + i, v);
-    else atomicAdd(a.grad + i, v);
+    if (grad) atomicAdd(grad + i, v);
+    else atomicAdd(sh_sums + n + i, v);
   }
 }
 
@@ -648,7 +649,7 @@ __global__ void __launch_bounds__(kAdjThreads, kAdjBlocks) k_adjoint(Scene s, Pa
       taken += unsigned(__popc(idle));
       if (taken >= a.flush) {
         taken -= a.flush;
-        pass_sums_on(a);
+        pass_sums_on(n_sums, a.sums == 2 ? nullptr : a.grad);
       }
       more = first + unsigned(__popc(idle)) < tasks;
       const unsigned t = first + unsigned(__popc(idle & ((1u << lane_id) - 1u)));
