@@ -313,18 +313,18 @@ typedef struct rm_batch_tuning {
   int32_t tile_shape;   /* pixels of a chunk: 0 a row segment, 1 a near-square block */
   int32_t grid_scale;   /* persistent grids: resident blocks per SM x this (1..4) */
   int32_t graph_waves;  /* waves per CUDA graph launch (even, 2..64); 0: no graph */
-  int32_t bvh_width;    /* 2: the binary BVH; 8: the 8-wide compressed BVH (collapsed per scene on first use) */
+  int32_t bvh_width;    /* 2: the scene's own (4-wide) BVH; 8: the 8-wide compressed BVH (collapsed per scene on first use) */
 } rm_batch_tuning;
 
 /* Render many images of (possibly different) scenes, views, resolutions,
  * sample counts and depths: on several streams, or together in one pool of
  * path slots (more than 32 images of fewer than 65,536 samples, those).  The
- * tuning applies to the pool.  Each image is
- * what the plain single-frame chain gives it: render_paths (K1) or the 8/32
- * lane kernel (K2) of pathtrace.metal:739-815 with the lane rule of
- * metal.mm:390-394, adaptive sampling and clamp, bit for bit equal to
- * rmcuda_render_scene_async with the same inputs (radiance, RGB8, samples
- * and RNG streams).  Items whose policy picks the ReSTIR chain are rejected
+ * tuning and the progress log concern the pool alone: a batch of larger or of
+ * fewer images is the same whatever the tuning.  Each image is what the plain
+ * single-frame chain gives it: render_paths (K1) or the 8/32 lane kernel (K2)
+ * of pathtrace.metal:739-815 with the lane rule of metal.mm:390-394, adaptive
+ * sampling and clamp, bit for bit equal to rmcuda_render_scene_async with the
+ * same inputs (radiance, RGB8, samples and RNG streams).  Items whose policy picks the ReSTIR chain are rejected
  * (set RM_FLAG_RESTIR_OFF, or restir_spatial 0).  Synchronous. */
 int rmcuda_render_batch(rmcuda_ctx* ctx, const rm_batch_item* items, int32_t n, char* err, size_t errcap);
 

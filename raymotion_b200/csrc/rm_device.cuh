@@ -391,8 +391,9 @@ struct Trav {
 // tail of the 720p ReSTIR frame 69 against 76 ms (three parts summed), a million
 // closest-hit queries 461 against 511 us (leaves of two triangles on both
 // sides).  The seven 128-bit loads in flight spill at the 48 registers of
-// k_wf_trace2 and k_restir_generate (frame 119 against 115 ms, generate 14.4
-// against 12.6), which keep the binary records.
+// k_wf_trace2 (frame 119 against 115 ms) and cost k_restir_generate, at 64, as
+// much (14.4 against 12.6): their rays, the latter's shadow rays, keep the
+// binary records.
 //
 // Pushes store all four words and advance the stack only for the hit ones: as
 // branches they split the warp (94 M against 52 M warp instructions for one
@@ -401,9 +402,10 @@ struct Trav {
 // (All before Tracer::trace made the traversal one copy per kernel.)
 //
 // Box test: Trav's, with the near and far bounds picked by the sign of i when
-// the node is read (near is lo for i >= 0) instead of by min / max; an axis
-// whose o i overflows culls nothing, as there.
-// A node on the way pushes three subtrees at most and lies one binary level or
+// the node is read (near is lo for i >= 0, so bounds are ordered in the nodes)
+// instead of by min / max; an axis whose o i overflows culls nothing, as there.
+//
+// The stack: a node on the way pushes three subtrees at most and lies one binary level or
 // more below the one before it (its children may include one it never opened).
 constexpr int kQuadStack = 3 * kStack + 4;
 
@@ -706,8 +708,8 @@ __device__ __forceinline__ TraceResult traverse(const Scene& s, float ox, float 
 }
 
 // One ray through the 8-wide BVH when the scene has one, else the 4-wide BVH
-// (the ray-query entry point; the wavefront trace kernels pick WTrav or QTrav
-// per launch instead).  Both give the same hits.
+// (the ray-query entry point; the wavefront trace kernels pick theirs per launch
+// instead).  Both give the same hits.
 template <bool kAnyHit>
 __device__ __forceinline__ TraceResult traverse_any(const Scene& s, float ox, float oy, float oz, float dx, float dy,
                                                     float dz, float tmax, uint32_t* err, uint32_t& n_nodes,

@@ -1,5 +1,9 @@
-// rm_quad.cu - the 4-wide BVH that every traversal but the no-allocation query
-// reads, collapsed from the binary child-pair records.
+// rm_quad.cu - the 4-wide BVH, collapsed from the binary child-pair records.
+//
+// The one-thread-per-path kernels, the adjoint, the batch and the ray queries
+// traverse it (QTrav); the wavefront's traversal, the shadow rays of a large
+// frame's ReSTIR candidates and of spatial reuse, and the no-allocation query
+// read the binary records (Trav).
 //
 // Traversal is bound by the chain of dependent node fetches of each ray (5 to
 // 6 of 32 lanes active, DRAM 3 % busy), so a node holds up to four children in
@@ -9,7 +13,7 @@
 // refit, where each child's box stands in the binary records (record << 1 |
 // slot, -1: no child).  Boxes are the binary records' own floats, so a ray's
 // hits are those of the binary BVH.  The format and its traversal are in
-// rm_device.cuh (Trav).
+// rm_device.cuh (QTrav).
 //
 // The collapse runs top-down, one launch per level without a read-back: a node
 // starts from the two children of its binary record and opens the internal

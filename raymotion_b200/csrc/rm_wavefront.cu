@@ -272,7 +272,9 @@ __global__ void __launch_bounds__(256) k_wf_init(Scene s, Params p, uint64_t see
 
 // Traversal of a queue of rays, one thread per ray (closest hit for extension
 // rays, pathtrace.metal:119-163; any hit for shadow rays, :164).  T is the
-// traversal (QTrav: 4-wide BVH, WTrav: 8-wide BVH) and E / kDepth its stack.
+// traversal (QTrav: 4-wide BVH, WTrav: 8-wide BVH) and E / kDepth its stack: the
+// launches of waves in separate steps and of the 8-wide BVH (k_wf_trace2
+// otherwise).
 // Finished extension rays are sorted into the shading queue of their surface
 // type.  (Persistent grids whose idle lanes claim new rays, per leaf-to-leaf
 // step or per node / triangle, measured 7-70 % slower on the 720p frame.)

@@ -111,13 +111,19 @@ void tile_shape(int lanes, int shape, int& tw, int& th) {
 // Images go through the plain frame's kernels (rm_paths.cu), on kStreams
 // streams: paths stay in registers there, where a wave of the pool stores and
 // reloads each path's state and ends with its slowest warps (eight images of
-// 45 k to 14.7 M samples 24.4 -> 12.0 ms; one of 64x36, 4 spp 1.4 -> 0.2; 64 of
-// 160x90, 16 spp 14.5 -> 10.3).  An image costs about 70 us of launches then,
-// which the pool pays once (2.2 to 2.5 ms a batch, then about 1.1 ns a sample),
-// so many small ones stay with the pool: more than kFewSmall images of fewer
-// than kOwnSamples samples (256 of 64x36, 4 spp 17.4 ms alone, 6.5 in the pool;
-// of 64x36, 16 spp 14.2 and 11.0; of 160x90, 4 spp 21.7 and 19.0; 64 of each 4.3
-// / 3.9, 3.6 / 4.4 and 5.4 / 6.7).
+// 45 k to 14.7 M samples 24.4 -> 11.8 ms; one of 64x36, 4 spp 1.4 -> 0.2).  An
+// image costs 40 to 55 us of launches then, which the pool pays once (2.4 ms a
+// batch), so many small ones stay with the pool: more than kFewSmall images of
+// fewer than kOwnSamples samples.  Alone / in the pool, ms:
+//               64x36, 4 spp   64x36, 16 spp   160x90, 4 spp
+//    33 images     1.3 / 2.4       1.2 / 2.5       1.7 / 3.7
+//    64            2.5 / 2.8       2.2 / 3.3       3.4 / 5.2
+//   128            4.9 / 3.5       4.5 / 5.4       6.8 / 8.5
+//   256            9.8 / 4.9       8.8 / 9.3      13.6 / 15.5
+// So the line is a cautious one: the pool pays from about 80 images of the
+// smallest size and from more than 256 of the others, which the count alone
+// does not tell apart; from 33 images to there a batch takes what it took when
+// all images went through the pool, and no more.
 constexpr double kOwnSamples = 65536.0;
 constexpr int kFewSmall = 32;
 constexpr long long kOwnChunk = 4ll << 20;  // samples whose values a stream holds (16 M: 11.9 ms)
