@@ -134,7 +134,11 @@ struct rmcuda_ctx {
   rmapi::ResSet rinit, rmerged, hres;
   rmd::DevBuf hdr, tmp_a, tmp_b, hist_col, rgb, dbg, hash_out;
   rmd::DevBuf ctr, err;
-  rmd::DevBuf paths;  // values, states, sums and lists of a plain frame (rm_paths.cu)
+  // values, states, sums and lists of a plain frame (rm_paths.cu); once a graph
+  // holds the buffer a larger one takes its place beside it (paths_kept)
+  rmd::DevBuf paths;
+  bool paths_in_graph = false;
+  std::vector<rmd::DevBuf> paths_kept;
   // pinned, a word per stream: the last chunk of a plain frame found without an open pixel
   unsigned long long* h_done = nullptr;
   unsigned long long ticket = 0;  // chunks so far
@@ -296,6 +300,8 @@ struct PathsRoom {
 // The next smaller room, for a workspace that the device had no memory for;
 // false when there is none.
 bool smaller_paths(rmcuda_ctx* c, PathsRoom& r);
+// The context's own workspace, of `bytes` at least.
+cudaError_t reserve_paths(rmcuda_ctx* c, size_t bytes);
 PathsPlan plan_paths(rmcuda_ctx* c, const rmd::Params& p, int lanes, const PathsRoom& r);
 // The plain chain of one image (rm_paths.cu), enqueued on t.stream.
 cudaError_t run_paths(rmcuda_ctx* c, const rmd::Scene& s, const rmd::Params& p, int lanes, uint64_t seed,

@@ -702,6 +702,30 @@ static PathsPlan plan_paths(rmcuda_ctx* c, const Params& p, int lanes, long long
   return q;
 }
 
+static bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
+
+// A stream that is being captured takes no new memory: what there is, or none.
+// Its graph keeps the address, so the buffer is never given back before the
+// context, and never grown.
+cudaError_t reserve_paths(rmcuda_ctx* c, size_t bytes) {
+  if (bytes == 0) return cudaSuccess;
+  if (capturing(c->stream)) {
+    if (bytes > c->paths.cap) return cudaErrorMemoryAllocation;
+    c->paths_in_graph = true;
+    return cudaSuccess;
+  }
+  if (bytes <= c->paths.cap) return cudaSuccess;
+  if (c->paths_in_graph) {
+    c->paths_kept.push_back(c->paths);
+    c->paths = DevBuf{};
+    c->paths_in_graph = false;
+  }
+  return c->paths.reserve(bytes);
+}
+
 bool smaller_paths(rmcuda_ctx* c, PathsRoom& r) {
   if (r.bare) return false;
   if (r.samples / 4 >= paths_one_wave(c->sms)) r.samples /= 4;
@@ -752,7 +776,7 @@ cudaError_t run_paths(rmcuda_ctx* c, const Scene& s, const Params& p, int lanes,
   // device it can save the rest: a long frame looks, without waiting, whether a
   // segment has found no open pixel (one even colour at 1,024 spp: 160x90 1.7 ->
   // 0.2 ms, 640x360 2.5 -> 1.9; a larger frame's launches are all out by then).
-  if (segs > kLookSegments && !c->h_done) {
+  if (segs > kLookSegments && !c->h_done && !capturing(t.stream)) {
     if (cudaMallocHost(reinterpret_cast<void**>(&c->h_done), kStreams * sizeof(*c->h_done)) != cudaSuccess) {
       cudaGetLastError();
       c->h_done = nullptr;
@@ -825,7 +849,7 @@ int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_co
     c->last_chain = pl.lanes;
     PathsRoom room{kPathChunk};
     PathsPlan q = plan_paths(c, p, pl.lanes, room);
-    while (q.bytes && (e = c->paths.reserve(q.bytes)) != cudaSuccess) {
+    while ((e = reserve_paths(c, q.bytes)) != cudaSuccess) {
       cudaGetLastError();
       if (!smaller_paths(c, room)) {
         msg = cuda_msg("Metal image buffer allocation failed", e);
@@ -968,12 +992,14 @@ int rmcuda_create(rmcuda_ctx** out, int device, char* err, size_t errcap) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = c->ctr.reserve(RM_STAGE_COUNT * 32 + 32);  // the adjoint's hand-out counter behind the stages'
   if (e == cudaSuccess) e = c->err.reserve(4);
+  if (e == cudaSuccess) e = c->paths.reserve(256);  // what a plain frame cannot do without
   if (e == cudaSuccess) e = cudaMemset(c->ctr.ptr, 0, RM_STAGE_COUNT * 32);
   if (e == cudaSuccess) e = cudaMemset(c->err.ptr, 0, 4);
   if (e != cudaSuccess) {
     set_err(err, errcap, cuda_msg("context creation failed", e));
     c->ctr.release();
     c->err.release();
+    c->paths.release();
     if (c->own) cudaStreamDestroy(c->own);
     pool_close(device);
     delete c;
@@ -994,6 +1020,7 @@ void rmcuda_destroy(rmcuda_ctx* c) {
   for (DevBuf* b : {&c->hdr, &c->tmp_a, &c->tmp_b, &c->hist_col, &c->rgb, &c->dbg, &c->hash_out, &c->ctr, &c->err,
                     &c->adj_scratch, &c->gen, &c->differ, &c->ctr_save, &c->paths})
     b->release();
+  for (DevBuf& b : c->paths_kept) b.release();
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   for (int h = 0; h < kStreams - 1; ++h) {
     if (c->side_stream[h]) cudaStreamDestroy(c->side_stream[h]);

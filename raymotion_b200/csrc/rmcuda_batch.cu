@@ -408,7 +408,7 @@ int run_own(rmcuda_ctx* c, const std::vector<BtJob>& jobs, std::string& msg) {
     // Short of memory, fewer streams, then smaller chunks.
     enough = true;
     for (int h = 0; h < parts && enough; ++h) {
-      const cudaError_t e = bytes[h] ? ws[h]->reserve(bytes[h]) : cudaSuccess;
+      const cudaError_t e = h == 0 ? reserve_paths(c, bytes[h]) : bytes[h] ? ws[h]->reserve(bytes[h]) : cudaSuccess;
       if (e == cudaSuccess) continue;
       cudaGetLastError();
       enough = false;

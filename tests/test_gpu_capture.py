@@ -1,0 +1,113 @@
+"""Frames captured into a CUDA graph: a context that has rendered a frame of the
+same size needs no memory and no wait for a plain frame of any other sample count,
+so the frame can be captured; its replay gives the frame."""
+import pytest
+
+from raymotion_b200 import Backend, RenderConfig, _abi
+from raymotion_b200.scenes import sized_field
+
+pytestmark = pytest.mark.gpu
+
+
+def _cfg(spp, adapt):
+    c = RenderConfig(width=320, height=180, spp=spp, max_bounces=4, restir_candidates=1, restir_spatial=0,
+                     flags=_abi.RM_FLAG_NO_ENV | _abi.RM_FLAG_DENOISE_OFF)
+    c.adapt_min, c.adapt_step = adapt
+    return c
+
+
+# one lane; 8 lanes and segments; more than eight segments; 32 lanes
+CASES = [(4, (16, 8)), (24, (16, 8)), (256, (16, 8)), (64, (0, 8))]
+
+
+@pytest.mark.parametrize("warm", [None, 1, 24], ids=["same", "after_1spp", "after_24spp"])
+@pytest.mark.parametrize("spp,adapt", CASES)
+def test_plain_frames(backend, spp, adapt, warm):
+    import torch
+    sb, cam, _ = sized_field(5, 3000, 64, 36, 1, 4)
+    sc = sb.pack()
+    out = torch.empty(320 * 180 * 3, device="cuda")
+    b = Backend(0)
+    scene = b.scene_create(sc)
+    try:
+        # (every kernel is loaded by a context of its own)
+        other = backend.scene_create(sc)
+        for s, a in [*CASES, (24, (16, 8))]:
+            backend.render_scene_async(other, cam, _cfg(s, a), 5, None, out.data_ptr())
+        small = _cfg(64, (32, 32))
+        small.width, small.height = 32, 18
+        backend.render_scene_async(other, cam, small, 5, None, out.data_ptr())
+        small.spp, small.adapt_min, small.adapt_step = 24, 16, 8
+        backend.render_scene_async(other, cam, small, 5, None, out.data_ptr())
+        backend.render_scene_async(other, cam, _cfg(spp, adapt), 5, None, out.data_ptr())
+        backend.sync()
+        backend.scene_destroy(other)
+        want = out.clone()
+        stream = torch.cuda.Stream()
+        b.set_stream(stream.cuda_stream)
+        # the frame's own images, which every call needs: by a frame of the same size
+        b.render_scene_async(scene, cam, _cfg(warm or 1, (16, 8)), 5, None, out.data_ptr())
+        if warm is None:
+            b.render_scene_async(scene, cam, _cfg(spp, adapt), 5, None, out.data_ptr())
+        b.sync()
+        out.zero_()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            b.render_scene_async(scene, cam, _cfg(spp, adapt), 5, None, out.data_ptr())
+        for _ in range(2):
+            out.zero_()
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+        del graph
+    finally:
+        torch.cuda.synchronize()
+        b.scene_destroy(scene)
+        b.close()
+
+
+@pytest.mark.parametrize("spp,adapt", CASES)
+def test_graphs_outlive_larger_frames(backend, spp, adapt):
+    """A graph keeps the workspace that it was captured with: a frame that needs a
+    larger one, and another context that takes freed memory, change nothing."""
+    import torch
+    sb, cam, _ = sized_field(5, 3000, 64, 36, 1, 4)
+    sc = sb.pack()
+    out, other_out = (torch.empty(320 * 180 * 3, device="cuda") for _ in range(2))
+    b, other = Backend(0), None
+    scene = b.scene_create(sc)
+    try:
+        stream = torch.cuda.Stream()
+        b.set_stream(stream.cuda_stream)
+        b.render_scene_async(scene, cam, _cfg(spp, adapt), 5, None, out.data_ptr())
+        b.sync()
+        want = out.clone()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            b.render_scene_async(scene, cam, _cfg(spp, adapt), 5, None, out.data_ptr())
+        b.render_scene_async(scene, cam, _cfg(320, (0, 8)), 6, None, out.data_ptr())
+        b.sync()
+        other = Backend(0)
+        theirs = other.scene_create(sc)
+        other.render_scene_async(theirs, cam, _cfg(64, (0, 8)), 7, None, other_out.data_ptr())
+        other.sync()
+        other_want = other_out.clone()
+        out.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+        other.render_scene_async(theirs, cam, _cfg(64, (0, 8)), 7, None, other_out.data_ptr())
+        other.sync()
+        assert torch.equal(other_out.view(torch.int32), other_want.view(torch.int32))
+        other.scene_destroy(theirs)
+        del graph
+    finally:
+        torch.cuda.synchronize()
+        b.scene_destroy(scene)
+        b.close()
+        if other:
+            other.close()
