@@ -138,6 +138,7 @@ struct rmcuda_ctx {
   // holds the buffer a larger one takes its place beside it (paths_kept)
   rmd::DevBuf paths;
   bool paths_in_graph = false;
+  unsigned captured_adjoints = 0;
   std::vector<rmd::DevBuf> paths_kept;
   // pinned, a word per stream: the last chunk of a plain frame found without an open pixel
   unsigned long long* h_done = nullptr;
@@ -272,6 +273,15 @@ Plan make_plan(const DevScene& sc, const rm_camera& cam, const rm_config& cfg);
 int enqueue_frame(rmcuda_ctx* c, DevScene& sc, const rm_camera& cam, const rm_config& cfg, uint64_t seed,
                   uint8_t* d_rgb, std::string& msg);
 int check_device_error(rmcuda_ctx* c, std::string& msg);
+
+inline bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
+
+// The adjoint's hand-out counters: the first for calls, which follow one another,
+// the others by turns for captured ones, whose graphs may run at the same time.
+constexpr unsigned kHandOuts = 1024;
 
 // How run_paths takes one image: its segments, and the layout of its workspace.
 struct PathsPlan {

@@ -85,6 +85,7 @@ int rmcuda_backward(rmcuda_ctx* c, const rmcuda_scene* scene, const rm_camera* c
   if (sc.n_materials <= 0) { set_err(err, errcap, "scene has no materials (rmcuda_scene_set_materials)"); return RM_ERR_INVALID; }
   // pixel lanes that the kernel has handed out
   unsigned* next = reinterpret_cast<unsigned*>(c->ctr.as<unsigned long long>() + 4 * RM_STAGE_COUNT);
+  if (capturing(c->stream)) next += 1 + c->captured_adjoints++ % (kHandOuts - 1);
   Plan pl = make_plan(sc, *cam, *cfg);
   if (pl.use_spatial) {
     // the ReSTIR chain: K5 replayed from the checkpoint the frame left in the

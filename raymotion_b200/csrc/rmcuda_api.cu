@@ -702,11 +702,6 @@ static PathsPlan plan_paths(rmcuda_ctx* c, const Params& p, int lanes, long long
   return q;
 }
 
-static bool capturing(cudaStream_t st) {
-  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
-}
-
 // A stream that is being captured takes no new memory: what there is, or none.
 // Its graph keeps the address, so the buffer is never given back before the
 // context, and never grown.
@@ -990,7 +985,8 @@ int rmcuda_create(rmcuda_ctx** out, int device, char* err, size_t errcap) {
   cudaError_t e = cudaSetDevice(device);
   pool_open(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = c->ctr.reserve(RM_STAGE_COUNT * 32 + 32);  // the adjoint's hand-out counter behind the stages'
+  // the adjoint's hand-out counters behind the stages'
+  if (e == cudaSuccess) e = c->ctr.reserve(RM_STAGE_COUNT * 32 + kHandOuts * sizeof(unsigned));
   if (e == cudaSuccess) e = c->err.reserve(4);
   if (e == cudaSuccess) e = c->paths.reserve(256);  // what a plain frame cannot do without
   if (e == cudaSuccess) e = cudaMemset(c->ctr.ptr, 0, RM_STAGE_COUNT * 32);

@@ -111,3 +111,45 @@ def test_graphs_outlive_larger_frames(backend, spp, adapt):
         b.close()
         if other:
             other.close()
+
+
+def test_gradients_of_two_graphs_at_the_same_time(backend):
+    """Two captured gradients hand out their pixel lanes apart from one another.
+    Rounding: the order of the additions, 2^-20 of the largest entry."""
+    import numpy as np
+    import torch
+
+    from raymotion_b200.scenes import inverse_scene
+    d = inverse_scene(4, n_spheres=10, n_dielectric=3, ground=20, width=128, height=128, spp=8, depth=5)
+    scene = backend.scene_create(d["scene"])
+    try:
+        backend.scene_set_materials(scene, d["params"], d["tri_material"])
+        dl = [torch.rand(128 * 128 * 3, device="cuda", generator=torch.Generator("cuda").manual_seed(k)) for k in (1, 2)]
+        grad = [torch.zeros(len(d["params"]) * 8, device="cuda") for _ in range(2)]
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        want, graphs = [], []
+        for k in range(2):
+            backend.set_stream(streams[k].cuda_stream)
+            torch.cuda.synchronize()
+            backend.backward(scene, d["camera"], d["config"], 5 + k, dl[k].data_ptr(), grad[k].data_ptr())
+            backend.sync()
+            want.append(grad[k].cpu().numpy())
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=streams[k], capture_error_mode="thread_local"):
+                backend.backward(scene, d["camera"], d["config"], 5 + k, dl[k].data_ptr(), grad[k].data_ptr())
+            graphs.append(g)
+        for _ in range(4):
+            for k in range(2):
+                grad[k].zero_()
+            torch.cuda.synchronize()
+            for k in range(2):
+                with torch.cuda.stream(streams[k]):
+                    graphs[k].replay()
+            torch.cuda.synchronize()
+            for k in range(2):
+                assert np.abs(grad[k].cpu().numpy() - want[k]).max() <= 2.0 ** -20 * np.abs(want[k]).max()
+        del graphs
+    finally:
+        torch.cuda.synchronize()
+        backend.set_stream(None)
+        backend.scene_destroy(scene)
