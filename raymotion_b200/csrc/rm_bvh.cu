@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <vector>
 
@@ -43,6 +44,7 @@ struct DevicePool {
   int users = 0;
   cudaMemPool_t pool = nullptr;
   cudaStream_t stream = nullptr;  // orders the pool's own allocations and frees; carries no work
+  void* anchor = nullptr;         // keeps the driver's block of small allocations, which wait_for_device takes from
 };
 DevicePool g_pools[kPoolDevices];
 
@@ -62,8 +64,13 @@ void pool_open(int device) {
   if (cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && supported &&
       cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) == cudaSuccess &&
       cudaMemPoolCreate(&p.pool, &props) == cudaSuccess &&
-      cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+      cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
+    if (cudaMalloc(&p.anchor, 256) != cudaSuccess) {
+      cudaGetLastError();
+      p.anchor = nullptr;
+    }
     return;
+  }
   // no pool here: cudaMalloc serves the buffers
   cudaGetLastError();
   if (p.pool) cudaMemPoolDestroy(p.pool);
@@ -78,6 +85,8 @@ void pool_close(int device) {
   std::lock_guard<std::mutex> lk(p.mu);
   if (--p.users > 0) return;
   if (p.stream) cudaStreamSynchronize(p.stream);
+  if (p.anchor) cudaFree(p.anchor);
+  p.anchor = nullptr;
   if (p.pool) cudaMemPoolDestroy(p.pool);
   if (p.stream) cudaStreamDestroy(p.stream);
   p.pool = nullptr;
@@ -109,25 +118,49 @@ cudaError_t DevBuf::reserve(size_t bytes) {
   return cudaSuccess;
 }
 
-void DevBuf::release() {
-  if (ptr && device >= 0) {
-    int now = device;
-    cudaGetDevice(&now);
-    if (now != device) cudaSetDevice(device);
-    // any stream of any context may still use the memory: wait, as cudaFree does
+namespace {
+
+// Waits for the device's work, as a cudaFree of a buffer does: any stream of any
+// context may still use pool memory that is given back.  By a cudaFree (5 us with
+// its cudaMalloc, 500 without the pool's anchor): cudaDeviceSynchronize is refused
+// while another thread captures a stream, and ends that capture.
+void wait_for_device(int device) {
+  int now = device;
+  cudaGetDevice(&now);
+  if (now != device) cudaSetDevice(device);
+  void* p = nullptr;
+  if (cudaMalloc(&p, 256) == cudaSuccess) {
+    cudaFree(p);
+  } else {
+    cudaGetLastError();
     cudaDeviceSynchronize();
-    DevicePool& p = g_pools[device];
-    std::lock_guard<std::mutex> lk(p.mu);
-    if (p.pool) cudaFreeAsync(ptr, p.stream);
-    else cudaFree(ptr);  // the pool went with its last context; its memory goes back here
-    if (now != device) cudaSetDevice(now);
-  } else if (ptr) {
-    cudaFree(ptr);
   }
-  ptr = nullptr;
-  cap = 0;
-  device = -1;
+  if (now != device) cudaSetDevice(now);
 }
+
+void give_back(DevBuf& b) {
+  if (b.ptr && b.device >= 0) {
+    DevicePool& p = g_pools[b.device];
+    std::lock_guard<std::mutex> lk(p.mu);
+    if (p.pool) cudaFreeAsync(b.ptr, p.stream);
+    else cudaFree(b.ptr);  // the pool went with its last context; its memory goes back here
+  } else if (b.ptr) {
+    cudaFree(b.ptr);
+  }
+  b = DevBuf{};
+}
+
+}  // namespace
+
+void release_all(std::initializer_list<DevBuf*> bufs) {
+  int waited = -1;
+  for (DevBuf* b : bufs) {
+    if (b->ptr && b->device >= 0 && b->device != waited) wait_for_device(waited = b->device);
+    give_back(*b);
+  }
+}
+
+void DevBuf::release() { release_all({this}); }
 
 namespace {
 

@@ -80,11 +80,10 @@ struct DevScene {
   DevBuf tri_mat, mats;
   int n_materials = 0;
   void release() {
-    for (DevBuf* b : {&tri_mat, &mats, &tris, &tris_in, &lights, &cdf, &texels, &lrec, &guide, &bvh.records, &bvh.parents, &bvh.counters,
-                      &bvh.order, &bvh.tgeo, &bvh.keys, &bvh.keys_alt, &bvh.vals_alt, &bvh.knodes, &bvh.kbox,
-                      &bvh.kcount, &bvh.ranges, &bvh.temp, &bvh.bounds, &bvh.depth, &bvh.quads, &bvh.qroots, &bvh.wnodes, &bvh.wtgeo,
-                      &bvh.wq})
-      b->release();
+    rmd::release_all({&tri_mat, &mats, &tris, &tris_in, &lights, &cdf, &texels, &lrec, &guide, &bvh.records,
+                      &bvh.parents, &bvh.counters, &bvh.order, &bvh.tgeo, &bvh.keys, &bvh.keys_alt, &bvh.vals_alt,
+                      &bvh.knodes, &bvh.kbox, &bvh.kcount, &bvh.ranges, &bvh.temp, &bvh.bounds, &bvh.depth, &bvh.quads,
+                      &bvh.qroots, &bvh.wnodes, &bvh.wtgeo, &bvh.wq});
     if (bvh.h_wcnt) cudaFreeHost(bvh.h_wcnt);
     bvh.h_wcnt = nullptr;
   }

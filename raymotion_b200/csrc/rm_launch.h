@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -243,6 +244,8 @@ struct DevBuf {
   void release();
   template <class T> T* as() const { return static_cast<T*>(ptr); }
 };
+// release() of them all, after one wait.
+void release_all(std::initializer_list<DevBuf*> bufs);
 
 // Device-resident BVH + triangle geometry of one scene.
 struct DevBvh {

@@ -153,3 +153,82 @@ def test_gradients_of_two_graphs_at_the_same_time(backend):
         torch.cuda.synchronize()
         backend.set_stream(None)
         backend.scene_destroy(scene)
+
+
+def _scenes_beside(backend_of_thread, sc, rounds):
+    """Create, grow and give back scenes in another thread; its errors."""
+    import threading
+    errors = []
+
+    def work():
+        try:
+            for _ in range(rounds):
+                h = backend_of_thread.scene_create(sc)
+                backend_of_thread.scene_destroy(h)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+    t = threading.Thread(target=work)
+    t.start()
+    return t, errors
+
+
+def test_memory_given_back_beside_a_capture(backend):
+    """Another thread's scenes come and go while this one captures a frame."""
+    import torch
+    sb, cam, _ = sized_field(5, 3000, 64, 36, 1, 4)
+    sc = sb.pack()
+    out = torch.empty(320 * 180 * 3, device="cuda")
+    b = Backend(0)
+    scene = backend.scene_create(sc)
+    try:
+        stream = torch.cuda.Stream()
+        backend.set_stream(stream.cuda_stream)
+        backend.render_scene_async(scene, cam, _cfg(4, (16, 8)), 5, None, out.data_ptr())
+        backend.sync()
+        want = out.clone()
+        out.zero_()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            backend.render_scene_async(scene, cam, _cfg(4, (16, 8)), 5, None, out.data_ptr())
+            t, errors = _scenes_beside(b, sc, 3)
+            t.join()
+        assert not errors
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+        del graph
+    finally:
+        torch.cuda.synchronize()
+        backend.set_stream(None)
+        backend.scene_destroy(scene)
+        b.close()
+
+
+def test_memory_given_back_beside_batches(backend):
+    """The batch's pool captures its waves; another context's scenes come and go."""
+    import torch
+
+    from raymotion_b200 import BatchItem
+    sb, cam, _ = sized_field(5, 3000, 64, 36, 1, 4)
+    sc = sb.pack()
+    cfg = _cfg(4, (0, 8))
+    cfg.width, cfg.height = 32, 18
+    b = Backend(0)
+    scene = backend.scene_create(sc)
+    outs = [torch.empty(32 * 18 * 3, device="cuda") for _ in range(40)]
+    items = [BatchItem(scene, cam, cfg, 9, None, o.data_ptr(), None) for o in outs]
+    try:
+        t, errors = _scenes_beside(b, sc, 60)
+        while t.is_alive():
+            for o in outs:
+                o.zero_()
+            torch.cuda.synchronize()
+            backend.render_batch(items)
+            assert len(backend.batch_log()) > 0
+            assert all(torch.equal(o, outs[0]) for o in outs) and outs[0].any()
+        t.join()
+        assert not errors
+    finally:
+        backend.scene_destroy(scene)
+        b.close()
